@@ -2100,17 +2100,12 @@ void create_batch(fea_batch* B, const fea_instance_desc* inst, int n) {
         H.h[i] = nullptr;
     }
     {  // tile-ELL layout of the stacked matrix
-        std::vector<int32_t> hrp(Nr + 1), hcol(nnz);
-        FEA_CUDA_TRY(cudaMemcpyAsync(hrp.data(), B->rp, sizeof(int32_t) * (Nr + 1), cudaMemcpyDeviceToHost, st));
-        if (nnz > 0)
-            FEA_CUDA_TRY(cudaMemcpyAsync(hcol.data(), B->col, sizeof(int32_t) * nnz, cudaMemcpyDeviceToHost, st));
-        FEA_CUDA_TRY(cudaStreamSynchronize(st));
-        if (build_tile_ell(hrp, hcol, Nr, sizeof(FV<R, 2>), kEllSmemBudget, B->ell, B->mem, st)) {
+        if (build_tile_ell(B->rp, B->col, Nr, sizeof(FV<R, 2>), kEllSmemBudget, B->ell, B->mem, st)) {
             B->As = B->mem.alloc<FV<R, 2>>(B->ell.E);
             fill_tile_ell<R, 2>(B->ell, (const FV<R, 2>*)B->A, (FV<R, 2>*)B->As, st);
             B->Ms = B->mem.alloc<R>(B->ell.E);
             fill_tile_ell<R, 1>(B->ell, (const FV<R, 1>*)B->M, (FV<R, 1>*)B->Ms, st);
-            if (build_tile_ell(hrp, hcol, Nr, sizeof(FV<R, 2>), kEllSmemBudget, B->ell_od, B->mem, st, true)) {
+            if (build_tile_ell(B->rp, B->col, Nr, sizeof(FV<R, 2>), kEllSmemBudget, B->ell_od, B->mem, st, true)) {
                 B->As_od = B->mem.alloc<FV<R, 2>>(B->ell_od.E);
                 fill_tile_ell<R, 2>(B->ell_od, (const FV<R, 2>*)B->A, (FV<R, 2>*)B->As_od, st);
             }

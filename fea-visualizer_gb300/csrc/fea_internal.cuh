@@ -34,6 +34,12 @@ int64_t build_idx_map(const uint8_t* ob, int64_t V, int bc, int32_t* idx, cudaSt
 void build_pattern(Pattern& P, DeviceArena& keep, const uint32_t* tri, int64_t T, const uint8_t* ob,
                    const int32_t* idx, int bc, int64_t N, cudaStream_t st);
 
+// ---- the solver's ordering (ordering.cu) ---------------------------------------------
+// inv[c] = unknown of solver row c, pos its inverse; rp: the pattern's row
+// pointers in unknown order, idx: node -> unknown (-1: none).
+void solver_order(const float* xyz, const int32_t* idx, int64_t V, const int32_t* rp, int64_t N, int32_t* inv,
+                  int32_t* pos, cudaStream_t st);
+
 // ---- tile-ELL operator layout (tile_ell.cu) ----------------------------------------
 // Tiles of kTileRows solver-order rows (one row per thread of a kBlock-thread
 // block), 32-row slices stored column by column, 16-bit tile-local column
@@ -56,13 +62,13 @@ struct TileEll {
     int32_t* emap = nullptr;       // [E] CSR slot of each entry, -1 for padding
     bool ok = false;
 };
-// From host copies of a solver-order CSR pattern.  Returns false (L.ok false)
+// From a solver-order CSR pattern on the device.  Returns false (L.ok false)
 // when a tile's halo does not fit the 16-bit indices or `smem_budget` bytes of
 // shared memory at fv_bytes per operand.
 // skip_diag: each row's diagonal entry is left out (a kernel that adds the
 // diagonal term from the row's own values reads the rest); no lcol2.
-bool build_tile_ell(const std::vector<int32_t>& rp, const std::vector<int32_t>& col, int64_t N, size_t fv_bytes,
-                    size_t smem_budget, TileEll& L, DeviceArena& keep, cudaStream_t st, bool skip_diag = false);
+bool build_tile_ell(const int32_t* rp, const int32_t* col, int64_t N, size_t fv_bytes, size_t smem_budget,
+                    TileEll& L, DeviceArena& keep, cudaStream_t st, bool skip_diag = false);
 // As[k] = A[emap[k]] (0 for padding): the layout's copy of operator values.
 template <typename R, int NF>
 void fill_tile_ell(const TileEll& L, const FV<R, NF>* A, FV<R, NF>* As, cudaStream_t st);

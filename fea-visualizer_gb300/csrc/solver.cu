@@ -193,7 +193,6 @@ struct fea_solver {
     void* Ms_ell = nullptr;                                    // tile-ELL copy of M
     TileEll ell_od;                                            // the layout without diagonal entries (ring kernels)
     void *S1d = nullptr, *S0d = nullptr, *S2d = nullptr;       // its copies of A1, A0, A2
-    std::vector<float> h_xyz;       // host copy of the points (ordering keys)
     uint8_t* adv_present = nullptr;
     Fields F;
     // loop state
@@ -286,70 +285,15 @@ void assemble(fea_solver* s) {
     s->op_dirty = true;
 }
 
-uint64_t spread3(uint32_t x) {  // 21 bits -> every third bit of 63
-    uint64_t v = x & 0x1fffffu;
-    v = (v | (v << 32)) & 0x1f00000000ffffull;
-    v = (v | (v << 16)) & 0x1f0000ff0000ffull;
-    v = (v | (v << 8)) & 0x100f00f00f00f00full;
-    v = (v | (v << 4)) & 0x10c30c30c30c30c3ull;
-    v = (v | (v << 2)) & 0x1249249249249249ull;
-    return v;
-}
-
-// The solver's ordering of the unknowns: sorted by the 63-bit Morton key of
-// their points (coordinates quantised to 21 bits over the bounding box), ties
-// by unknown number, then by stored-entry count within each tile of
-// kTileRows rows.  Neighbouring points get nearby numbers, so a tile is a
-// compact patch whose rows mostly reference each other.  Computed on the host
-// once per mesh and boundary condition.
+// The solver's ordering (ordering.cu) and the pattern in it.
 void build_ordering(fea_solver* s) {
     cudaStream_t st = s->stream;
     const int64_t V = s->V, N = s->N;
-    std::vector<int32_t> idx(V);
-    FEA_CUDA_TRY(cudaMemcpyAsync(idx.data(), s->idx, sizeof(int32_t) * V, cudaMemcpyDeviceToHost, st));
-    FEA_CUDA_TRY(cudaStreamSynchronize(st));
-    float lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
-    for (int d = 0; d < 3; d++) {
-        lo[d] = hi[d] = V ? s->h_xyz[d] : 0.f;
-        for (int64_t i = 0; i < V; i++) {
-            lo[d] = std::min(lo[d], s->h_xyz[3 * i + d]);
-            hi[d] = std::max(hi[d], s->h_xyz[3 * i + d]);
-        }
-    }
-    std::vector<std::pair<uint64_t, int32_t>> key;
-    key.reserve(N);
-    for (int64_t i = 0; i < V; i++) {
-        if (idx[i] < 0) continue;
-        uint64_t m = 0;
-        for (int d = 0; d < 3; d++) {
-            const double ext = (double)hi[d] - (double)lo[d];
-            double t = ext > 0 ? ((double)s->h_xyz[3 * i + d] - lo[d]) / ext : 0.0;
-            t = t < 0 ? 0 : (t > 1 ? 1 : t);
-            m |= spread3((uint32_t)(t * 2097151.0)) << d;
-        }
-        key.emplace_back(m, idx[i]);
-    }
-    std::sort(key.begin(), key.end());
-    // within each tile of kTileRows rows, rows by stored-entry count, so the
-    // 32-row slices of the tile-ELL layout carry little padding (the tile's
-    // row set, hence its locality, is that of the Morton order)
-    std::vector<int32_t> rp(N + 1);
-    FEA_CUDA_TRY(cudaMemcpyAsync(rp.data(), s->P.row_ptr, sizeof(int32_t) * (N + 1), cudaMemcpyDeviceToHost, st));
-    FEA_CUDA_TRY(cudaStreamSynchronize(st));
-    std::vector<int32_t> pos(N), inv(N);
-    for (int64_t c = 0; c < N; c++) inv[c] = key[c].second;
-    for (int64_t t0 = 0; t0 < N; t0 += kTileRows)
-        std::stable_sort(inv.begin() + t0, inv.begin() + std::min<int64_t>(N, t0 + kTileRows),
-                         [&](int32_t a, int32_t b) { return rp[a + 1] - rp[a] < rp[b + 1] - rp[b]; });
-    for (int64_t c = 0; c < N; c++) pos[inv[c]] = (int32_t)c;
     s->pos = s->mat_mem.alloc<int32_t>(N);
     s->inv = s->mat_mem.alloc<int32_t>(N);
     s->emap = s->mat_mem.alloc<int32_t>(s->P.nnz);
     s->idx_c = s->mat_mem.alloc<int32_t>(V);
-    if (N > 0) {
-        FEA_CUDA_TRY(cudaMemcpyAsync(s->pos, pos.data(), sizeof(int32_t) * N, cudaMemcpyHostToDevice, st));
-        FEA_CUDA_TRY(cudaMemcpyAsync(s->inv, inv.data(), sizeof(int32_t) * N, cudaMemcpyHostToDevice, st));
-    }
+    solver_order(s->xyz, s->idx, V, s->P.row_ptr, N, s->inv, s->pos, st);
     k_compose_idx<<<launch_grid(V), kBlock, 0, st>>>(s->idx, s->pos, V, s->idx_c);
     FEA_CHECK_LAUNCH();
     build_permuted(s->P, s->pos, s->inv, s->Pc, s->emap, s->mat_mem, st);
@@ -376,11 +320,7 @@ void build_context(fea_solver* s) {
     const int64_t N = s->N, nnz = s->P.nnz, T = s->T;
     build_ordering(s);
     {
-        std::vector<int32_t> rp(N + 1), col(nnz);
-        FEA_CUDA_TRY(cudaMemcpyAsync(rp.data(), s->Pc.row_ptr, sizeof(int32_t) * (N + 1), cudaMemcpyDeviceToHost, st));
-        if (nnz > 0)
-            FEA_CUDA_TRY(cudaMemcpyAsync(col.data(), s->Pc.col, sizeof(int32_t) * nnz, cudaMemcpyDeviceToHost, st));
-        FEA_CUDA_TRY(cudaStreamSynchronize(st));
+        const int32_t *rp = s->Pc.row_ptr, *col = s->Pc.col;
         build_tile_ell(rp, col, N, 2 * rsize(s), kEllSmemBudget, s->ell, s->mat_mem, st);
         if (s->ell.ok) {
             s->S1 = ralloc(s->mat_mem, s, s->ell.E);
@@ -1405,7 +1345,6 @@ int fea_create(const float* vertices, int64_t V, const uint32_t* triangles, int6
     s->T = T;
     if (params) s->prm = *params;
     else fea_params_default(&s->prm);
-    s->h_xyz.assign(vertices, vertices + 3 * V);
     s->xyz = s->mesh_mem.alloc<float>(3 * V);
     s->tri = s->mesh_mem.alloc<uint32_t>(3 * T);
     s->ob = s->mesh_mem.alloc<uint8_t>(V);
