@@ -1,6 +1,7 @@
 // fea_internal.cuh -- types shared by the translation units of libfea_gb300.
 #pragma once
 
+#include <array>
 #include <vector>
 
 #include "fea_common.cuh"
@@ -62,16 +63,53 @@ struct TileEll {
     int32_t* emap = nullptr;       // [E] CSR slot of each entry, -1 for padding
     bool ok = false;
 };
+// Rows of a pattern given anew: row r with of[r] >= 0 holds the entries
+// off[of[r]] .. off[of[r] + 1] of col (sorted) and slot (their emap numbers).
+struct ModRows {
+    const int32_t *of = nullptr, *off = nullptr, *col = nullptr, *slot = nullptr;
+};
 // From a solver-order CSR pattern on the device.  Returns false (L.ok false)
 // when a tile's halo does not fit the 16-bit indices or `smem_budget` bytes of
 // shared memory at fv_bytes per operand.
 // skip_diag: each row's diagonal entry is left out (a kernel that adds the
 // diagonal term from the row's own values reads the rest); no lcol2.
+// mod: rows whose entries replace the pattern's (null: none).
 bool build_tile_ell(const int32_t* rp, const int32_t* col, int64_t N, size_t fv_bytes, size_t smem_budget,
-                    TileEll& L, DeviceArena& keep, cudaStream_t st, bool skip_diag = false);
-// As[k] = A[emap[k]] (0 for padding): the layout's copy of operator values.
+                    TileEll& L, DeviceArena& keep, cudaStream_t st, bool skip_diag = false,
+                    const ModRows* mod = nullptr);
+// As[k] = A[emap[k]] (0 for padding): the layout's copy of operator values;
+// entries numbered from nnz on come from X.
 template <typename R, int NF>
-void fill_tile_ell(const TileEll& L, const FV<R, NF>* A, FV<R, NF>* As, cudaStream_t st);
+void fill_tile_ell(const TileEll& L, const FV<R, NF>* A, FV<R, NF>* As, cudaStream_t st,
+                   const FV<R, NF>* X = nullptr, int64_t nnz = INT32_MAX);
+
+// ---- stiff groups (stiff.cu) --------------------------------------------------------
+struct StiffGroups {
+    int n = 0;                 // groups
+    int nx = 0;                // entries of A' = Q^T A Q that differ from A's
+    int32_t* mem = nullptr;    // [4 n] members (solver rows), -1 unused
+    int32_t* where = nullptr;  // [N] 4 * group + place of a member, -1 elsewhere
+    int32_t* xr = nullptr;     // [nx] row and column of each such entry
+    int32_t* xc = nullptr;
+};
+// One operator's change of basis.
+struct StiffBasis {
+    double* Q = nullptr;   // [n * fields * 16] eigenvectors: Q[4 member + place]
+    void* X = nullptr;     // [nx] values of A' (handle type, per field)
+    void* dinv = nullptr;  // inverse diagonal of A'
+};
+// Groups of the pattern P's unknowns by its stiffness matrix K, four unknowns
+// each (-1 unused).
+std::vector<std::array<int32_t, 4>> find_stiff_groups(const Pattern& P, const double* K, cudaStream_t st);
+bool stiff_groups_wanted(int64_t N);  // whether a mesh of N unknowns is searched for them
+// The groups in solver order and the rows of Pc's pattern that A' changes
+// (M.of etc. in `keep`).  False, nothing set, when a row involved is too long.
+bool plan_stiff_rows(const std::vector<std::array<int32_t, 4>>& unknowns, const Pattern& Pc, const int32_t* pos,
+                     StiffGroups& G, ModRows& M, DeviceArena& keep, cudaStream_t st);
+// Q, X and dinv of the operator A (solver order; dinv: its inverse diagonal).
+template <typename R, int NF>
+void update_stiff_basis(const StiffGroups& G, const Pattern& Pc, const FV<R, NF>* A, const FV<R, NF>* dinv,
+                        const StiffBasis& B, cudaStream_t st);
 
 // ---- assembly (assemble.cu) ---------------------------------------------------
 template <typename R>
@@ -192,11 +230,22 @@ struct StepArgs {
     // The same layout without the diagonal entries (ring kernels, when built):
     // the iteration adds the diagonal term A_ii u'_i = r'_i from the row's
     // own residual (u' = D^-1 r'), so the operator stream carries one entry
-    // less per row.  Same halo lists.  Null: the full layout above.
+    // less per row.  Null: the full layout above.
     const FV<R, NF>* As_od;
     const uint16_t* lcol_od;
     const int32_t* slice_off_od;
-    int emax_od;
+    const int32_t* halo_off_od;
+    const int32_t* halo_col_od;
+    int hmax_od, emax_od;
+    // Stiff groups (ring kernels; stiff.cu): the diagonal-free layout holds A' =
+    // Q^T A Q and dinv_it its inverse diagonal; k_stiff_in moves the groups'
+    // rows of a solve's start into the basis and k_stiff_out its result back.
+    const FV<R, NF>* dinv_it;  // inverse diagonal of the iterated operator
+    int ngrp;
+    const int32_t* grp_mem;
+    const double* grp_Q;
+    FV<R, NF>* grp_x0;  // [4 ngrp] the members' start values during a solve
+    int* grp_in;        // 1 while a solve's rows are in the basis
     const R* Ms;  // tile-ELL copy of M (the staged Gray-Scott right-hand side), or null
     const StepParams* prm;
     CgState* cg;
@@ -267,6 +316,8 @@ int max_grid_blocks();
 // CG variants whose iteration kernels finish the previous launch's iteration
 // at their start (deferred finish; see StepArgs::defer).
 constexpr bool is_deferred_variant(int l) { return l >= 10 && l <= 15 && l != 12; }
+// The ring variants, whose iteration runs in the stiff groups' basis.
+constexpr bool is_ring_variant(int l) { return l == 14 || l == 15; }
 
 // ---- adjoint of the explicit advection-diffusion step (adjoint.cu) ----------------
 // lam = M (u - t), *J = 1/2 (u - t).lam  (exact accumulators; one block-partial

@@ -193,6 +193,13 @@ struct fea_solver {
     void* Ms_ell = nullptr;                                    // tile-ELL copy of M
     TileEll ell_od;                                            // the layout without diagonal entries (ring kernels)
     void *S1d = nullptr, *S0d = nullptr, *S2d = nullptr;       // its copies of A1, A0, A2
+    StiffGroups grp;                // groups tied by nearly degenerate triangles (stiff.cu)
+    TileEll ell_st;                 // the diagonal-free layout of A' = Q^T A Q
+    void *S1s = nullptr, *S0s = nullptr, *S2s = nullptr;       // its copies of A1', A0', A2'
+    StiffBasis B1, B0, B2;          // the bases of A1, A0, A2
+    void* grp_x0 = nullptr;         // the groups' start values during a solve
+    int* grp_in = nullptr;
+    bool diagonal_only = false;     // solves without the stiff groups (DiagonalOnly)
     uint8_t* adv_present = nullptr;
     Fields F;
     // loop state
@@ -206,6 +213,7 @@ struct fea_solver {
     bool stream_mode = false;  // FEA_LAUNCH_MODE=stream: kernel-by-kernel launches
     RunState* h_run = nullptr;  // pinned
     StepGraph graph, init_graph;
+    StepGraph diag_graph;  // the step graph without the stiff groups
     int lanes = 8;  // CG kernel variant: 0/1 tile-ELL (8/4 entries prefetched), 2/3 streamed (stages), 4/8/16 CSR window
     bool op_dirty = true;
     int op_kind = -1;
@@ -222,11 +230,10 @@ namespace {
 
 size_t rsize(const fea_solver* s) { return s->precision == FEA_FP64 ? 8 : 4; }
 
-// Entries of the largest tile the ring kernels stream (the diagonal-free
-// layout when it was built).
-// The widest tile of the ring kernels' layouts: the set-up product streams
-// the full layout, the iteration the one without the diagonal.
-int ring_emax(const fea_solver* s) { return s->ell.emax; }
+// The widest tile and halo of the ring kernels' layouts: the once-per-step
+// passes stream the full layout, the iteration one without the diagonal.
+int ring_emax(const fea_solver* s) { return std::max(s->ell.emax, s->ell_st.emax); }
+int ring_hmax(const fea_solver* s) { return std::max(s->ell.hmax, s->ell_st.hmax); }
 
 int64_t pad_tiles(int64_t n) { return ceil_div(n, kTileRows) * kTileRows; }
 
@@ -299,10 +306,45 @@ void build_ordering(fea_solver* s) {
     build_permuted(s->P, s->pos, s->inv, s->Pc, s->emap, s->mat_mem, st);
 }
 
+// The stiff groups of the mesh and the diagonal-free layout in their basis:
+// A' has the pattern of A with the groups' rows and columns filled in.
+// False, and no groups, when there are none or the layout does not fit.
+bool build_stiff_layout(fea_solver* s) {
+    cudaStream_t st = s->stream;
+    const int64_t N = s->N;
+    if (!stiff_groups_wanted(N)) return false;
+    // the groups follow the mesh alone: K without the per-element diffusivity
+    element_matrices<double>(s->xyz, s->tri, s->T, 0, s->prm.advdiff_velocity, nullptr, s->Kloc, s->Mloc, s->Aloc, st);
+    ordered_sum<double>(s->P, s->Kloc, nullptr, s->K64, st);
+    const std::vector<std::array<int32_t, 4>> groups = find_stiff_groups(s->P, s->K64, st);
+    StiffGroups G;
+    ModRows mod;
+    if (groups.empty() || !plan_stiff_rows(groups, s->Pc, s->pos, G, mod, s->mat_mem, st) ||
+        !build_tile_ell(s->Pc.row_ptr, s->Pc.col, N, 2 * rsize(s), kEllSmemBudget, s->ell_st, s->mat_mem, st, true,
+                        &mod))
+        return false;
+    s->grp = G;
+    s->S1s = ralloc(s->mat_mem, s, s->ell_st.E);
+    s->S0s = ralloc(s->mat_mem, s, s->ell_st.E);
+    s->S2s = ralloc(s->mat_mem, s, 2 * s->ell_st.E);
+    const std::pair<StiffBasis*, int> bases[3] = {{&s->B1, 1}, {&s->B0, 1}, {&s->B2, 2}};
+    for (const auto& b : bases) {
+        b.first->Q = s->mat_mem.alloc<double>(16 * (int64_t)G.n * b.second);
+        b.first->X = ralloc(s->mat_mem, s, (int64_t)G.nx * b.second);
+        b.first->dinv = ralloc(s->mat_mem, s, pad_tiles(N) * b.second);
+        FEA_CUDA_TRY(cudaMemsetAsync(b.first->dinv, 0, rsize(s) * (size_t)(pad_tiles(N) * b.second), st));
+    }
+    s->grp_x0 = ralloc(s->mat_mem, s, 8 * (int64_t)G.n);
+    s->grp_in = s->mat_mem.alloc<int>(1);
+    FEA_CUDA_TRY(cudaMemsetAsync(s->grp_in, 0, sizeof(int), st));
+    return true;
+}
+
 // FEMContext::update_boundary_conditions + assemble_matrices and the state.
 void build_context(fea_solver* s) {
     s->graph.destroy();
     s->init_graph.destroy();
+    s->diag_graph.destroy();
     s->mat_mem.release();
     s->P = Pattern{};
     s->Pc = Pattern{};
@@ -312,6 +354,10 @@ void build_context(fea_solver* s) {
     s->S1 = s->S0 = s->S2 = nullptr;
     s->S1d = s->S0d = s->S2d = nullptr;
     s->Ms_ell = nullptr;
+    s->grp = StiffGroups{};
+    s->ell_st = TileEll{};
+    s->S1s = s->S0s = s->S2s = nullptr;
+    s->B1 = s->B0 = s->B2 = StiffBasis{};
     s->F = Fields{};
     cudaStream_t st = s->stream;
     s->idx = s->mat_mem.alloc<int32_t>(s->V);
@@ -319,6 +365,12 @@ void build_context(fea_solver* s) {
     build_pattern(s->P, s->mat_mem, s->tri, s->T, s->ob, s->idx, s->bc, s->N, st);
     const int64_t N = s->N, nnz = s->P.nnz, T = s->T;
     build_ordering(s);
+    s->Kloc = s->mat_mem.alloc<double>(9 * T);
+    s->Mloc = s->mat_mem.alloc<double>(9 * T);
+    s->Aloc = s->mat_mem.alloc<double>(9 * T);
+    s->K64 = s->mat_mem.alloc<double>(nnz);
+    s->M64 = s->mat_mem.alloc<double>(nnz);
+    s->Adv64 = s->mat_mem.alloc<double>(nnz);
     {
         const int32_t *rp = s->Pc.row_ptr, *col = s->Pc.col;
         build_tile_ell(rp, col, N, 2 * rsize(s), kEllSmemBudget, s->ell, s->mat_mem, st);
@@ -332,6 +384,7 @@ void build_context(fea_solver* s) {
                 s->S0d = ralloc(s->mat_mem, s, s->ell_od.E);
                 s->S2d = ralloc(s->mat_mem, s, 2 * s->ell_od.E);
             }
+            build_stiff_layout(s);
         }
         // both field counts fit when the two-field stages do
         const size_t stage = s->precision == FEA_FP64 ? stream_stage_bytes<double, 2>(s->ell.emax, s->ell.hmax)
@@ -341,20 +394,15 @@ void build_context(fea_solver* s) {
         // its stages fit, else the streamed deferred-finish kernel with as
         // many stages as fit, else the tile-ELL kernel, else windowed CSR
         const int remax = ring_emax(s);
-        const size_t ring = s->precision == FEA_FP64 ? ring_smem_bytes<double, 2>(remax, s->ell.hmax, 3)
-                                                     : ring_smem_bytes<float, 2>(remax, s->ell.hmax, 3);
+        const int rhmax = ring_hmax(s);
+        const size_t ring = s->precision == FEA_FP64 ? ring_smem_bytes<double, 2>(remax, rhmax, 3)
+                                                     : ring_smem_bytes<float, 2>(remax, rhmax, 3);
         s->lanes = !s->ell.ok ? 8
                    : ring <= kStreamSmemLimit ? 14
                    : s->stream_stages >= 3    ? 11
                    : s->stream_stages >= 2    ? 10
                                               : 0;
     }
-    s->Kloc = s->mat_mem.alloc<double>(9 * T);
-    s->Mloc = s->mat_mem.alloc<double>(9 * T);
-    s->Aloc = s->mat_mem.alloc<double>(9 * T);
-    s->K64 = s->mat_mem.alloc<double>(nnz);
-    s->M64 = s->mat_mem.alloc<double>(nnz);
-    s->Adv64 = s->mat_mem.alloc<double>(nnz);
     if (s->precision == FEA_FP64) {
         s->K = s->K64;
         s->M = s->M64;
@@ -410,6 +458,14 @@ void build_context(fea_solver* s) {
     s->acc_valid = false;
     assemble(s);
     FEA_CUDA_TRY(cudaStreamSynchronize(st));
+}
+
+// Whether the current equation's solves run in the stiff groups' basis.
+// Implicit advection-diffusion does not: its operator is not symmetric, CG
+// may break down on it, and it keeps the iteration it had.
+bool stiff_solves(const fea_solver* s) {
+    const bool symmetric = s->prm.equation != FEA_ADVECTION_DIFFUSION || s->prm.advection_scheme == 1;
+    return s->grp.n > 0 && is_ring_variant(s->lanes) && !s->diagonal_only && symmetric;
 }
 
 // r, w and s of the Chronopoulos-Gear iteration, two buffers each, carved
@@ -468,14 +524,31 @@ StepArgs<R, NF> make_args(fea_solver* s, bool init_op) {
         a.hmax = s->ell.hmax;
         a.emax = s->ell.emax;
         a.Ms = (const R*)s->Ms_ell;
-        if (s->ell_od.ok) {
-            if constexpr (NF == 1) a.As_od = (const FV<R, 1>*)(init_op ? s->S0d : s->S1d);
-            else a.As_od = (const FV<R, 2>*)s->S2d;
-            a.lcol_od = s->ell_od.lcol;
-            a.slice_off_od = s->ell_od.slice_off;
-            a.emax_od = s->ell_od.emax;
+        const bool stiff = stiff_solves(s);
+        const TileEll& od = stiff ? s->ell_st : s->ell_od;
+        if (od.ok) {
+            if constexpr (NF == 1)
+                a.As_od = (const FV<R, 1>*)(stiff ? (init_op ? s->S0s : s->S1s) : (init_op ? s->S0d : s->S1d));
+            else
+                a.As_od = (const FV<R, 2>*)(stiff ? s->S2s : s->S2d);
+            a.lcol_od = od.lcol;
+            a.slice_off_od = od.slice_off;
+            a.halo_off_od = od.halo_off;
+            a.halo_col_od = od.halo_col;
+            a.hmax_od = od.hmax;
+            a.emax_od = od.emax;
+        }
+        if (stiff) {
+            const StiffBasis& B = NF == 2 ? s->B2 : init_op ? s->B0 : s->B1;
+            a.dinv_it = (const FV<R, NF>*)B.dinv;
+            a.ngrp = s->grp.n;
+            a.grp_mem = s->grp.mem;
+            a.grp_Q = B.Q;
+            a.grp_x0 = (FV<R, NF>*)s->grp_x0;
+            a.grp_in = s->grp_in;
         }
     }
+    if (!a.dinv_it) a.dinv_it = a.dinv;
     a.prm = s->d_prm;
     a.cg = s->d_cg + 1;
     a.cg_alt = s->d_cg;
@@ -531,6 +604,17 @@ void upload_params(fea_solver* s) {
     FEA_CUDA_TRY(cudaStreamSynchronize(s->stream));
 }
 
+// The iteration's copies of an operator A: the diagonal-free layout Sd of A
+// itself and Ss of A' = Q^T A Q (with stiff groups).
+template <typename R, int NF>
+void fill_iterated(fea_solver* s, const void* A, const void* dinv, void* Sd, const StiffBasis& B, void* Ss) {
+    const auto* Av = (const FV<R, NF>*)A;
+    fill_tile_ell<R, NF>(s->ell_od, Av, (FV<R, NF>*)Sd, s->stream);
+    if (s->grp.n == 0) return;
+    update_stiff_basis<R, NF>(s->grp, s->Pc, Av, (const FV<R, NF>*)dinv, B, s->stream);
+    fill_tile_ell<R, NF>(s->ell_st, Av, (FV<R, NF>*)Ss, s->stream, (const FV<R, NF>*)B.X, s->P.nnz);
+}
+
 // Operator coefficients (the float parameters widened to double; the
 // operator is evaluated in FP64 and rounded once to the handle's type).
 template <typename R>
@@ -544,7 +628,7 @@ void update_operator(fea_solver* s, int kind) {
         combine_operator<R, 2>(s->Pc, s->emap, s->M64, s->K64, s->Adv64, c, (FV<R, 2>*)s->F.A2, (FV<R, 2>*)s->F.d2,
                                s->stream);
         fill_tile_ell<R, 2>(s->ell, (const FV<R, 2>*)s->F.A2, (FV<R, 2>*)s->S2, s->stream);
-        fill_tile_ell<R, 2>(s->ell_od, (const FV<R, 2>*)s->F.A2, (FV<R, 2>*)s->S2d, s->stream);
+        fill_iterated<R, 2>(s, s->F.A2, s->F.d2, s->S2d, s->B2, s->S2s);
     } else {
         OpCoef<1> c{};
         c.f[0] = {dt, 0.0, 1.0, 0.0};
@@ -568,12 +652,12 @@ void update_operator(fea_solver* s, int kind) {
             combine_operator<R, 1>(s->Pc, s->emap, s->M64, s->K64, s->Adv64, m, (FV<R, 1>*)s->F.A0, (FV<R, 1>*)s->F.d0,
                                    s->stream);
             fill_tile_ell<R, 1>(s->ell, (const FV<R, 1>*)s->F.A0, (FV<R, 1>*)s->S0, s->stream);
-            fill_tile_ell<R, 1>(s->ell_od, (const FV<R, 1>*)s->F.A0, (FV<R, 1>*)s->S0d, s->stream);
+            fill_iterated<R, 1>(s, s->F.A0, s->F.d0, s->S0d, s->B0, s->S0s);
         }
         combine_operator<R, 1>(s->Pc, s->emap, s->M64, s->K64, s->Adv64, c, (FV<R, 1>*)s->F.A1, (FV<R, 1>*)s->F.d1,
                                s->stream);
         fill_tile_ell<R, 1>(s->ell, (const FV<R, 1>*)s->F.A1, (FV<R, 1>*)s->S1, s->stream);
-        fill_tile_ell<R, 1>(s->ell_od, (const FV<R, 1>*)s->F.A1, (FV<R, 1>*)s->S1d, s->stream);
+        fill_iterated<R, 1>(s, s->F.A1, s->F.d1, s->S1d, s->B1, s->S1s);
     }
 }
 
@@ -600,6 +684,16 @@ struct GuessOff {
         cudaMemsetAsync(&s->d_run->prev_valid, 0, sizeof(int), s->stream);
         cudaStreamSynchronize(s->stream);
     }
+};
+
+// Solves without the stiff groups while it lives: the FP32 Gray-Scott adjoint
+// returns FP64 parameter gradients, sums over FP32 fields whose last digits
+// follow the iteration's rounding, and keeps the diagonal iteration it was
+// validated with.
+struct DiagonalOnly {
+    fea_solver* s;
+    DiagonalOnly(fea_solver* h, bool on) : s(h) { s->diagonal_only = on; }
+    ~DiagonalOnly() { s->diagonal_only = false; }
 };
 
 template <typename R>
@@ -657,8 +751,9 @@ void advance(fea_solver* s, int64_t nsteps) {
         run_graph<R, 1>(s, s->init_graph, EQ_NEWMARK_INIT, true, 1);
         s->acc_valid = true;
     }
-    if (two_fields(kind)) run_graph<R, 2>(s, s->graph, kind, false, nsteps);
-    else run_graph<R, 1>(s, s->graph, kind, false, nsteps);
+    StepGraph& graph = stiff_solves(s) ? s->graph : s->diag_graph;
+    if (two_fields(kind)) run_graph<R, 2>(s, graph, kind, false, nsteps);
+    else run_graph<R, 1>(s, graph, kind, false, nsteps);
 }
 
 void check_handle(const fea_solver* s) {
@@ -875,6 +970,7 @@ double adjoint_gs_core(fea_solver* s, const FV<R, 2>* x0, const FV<R, 2>* t, int
         throw Error{FEA_ERR_STATE};
     }
     const GuessOff guess_off(s);  // recomputed forward states must equal the forward sweep's
+    const DiagonalOnly diagonal(s, sizeof(R) == 4 && s->grp.n > 0);
     cudaStream_t st = s->stream;
     const int64_t N = s->N;
     const size_t xb = sizeof(FV<R, 2>) * (size_t)N;
@@ -1397,6 +1493,7 @@ int fea_destroy(fea_solver* s) {
     if (s->stream) cudaStreamSynchronize(s->stream);
     s->graph.destroy();
     s->init_graph.destroy();
+    s->diag_graph.destroy();
     s->mat_mem.release();
     s->run_mem.release();
     s->mesh_mem.release();
@@ -1783,8 +1880,8 @@ static int variant_check(const fea_solver* s, int l) {
     if (!csr && !s->ell.ok) return FEA_ERR_UNSUPPORTED;
     if (s->stream_stages < stages) return FEA_ERR_UNSUPPORTED;
     if (ring) {
-        const size_t need = s->precision == FEA_FP64 ? ring_smem_bytes<double, 2>(ring_emax(s), s->ell.hmax, ring)
-                                                     : ring_smem_bytes<float, 2>(ring_emax(s), s->ell.hmax, ring);
+        const size_t need = s->precision == FEA_FP64 ? ring_smem_bytes<double, 2>(ring_emax(s), ring_hmax(s), ring)
+                                                     : ring_smem_bytes<float, 2>(ring_emax(s), ring_hmax(s), ring);
         if (need > kStreamSmemLimit) return FEA_ERR_UNSUPPORTED;
     }
     return FEA_OK;

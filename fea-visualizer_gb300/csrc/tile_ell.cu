@@ -27,13 +27,13 @@ namespace {
 
 template <typename R, int NF>
 __global__ void k_fill_tile_ell(int64_t E, const int32_t* __restrict__ emap, const FV<R, NF>* __restrict__ A,
-                                FV<R, NF>* As) {
+                                const FV<R, NF>* __restrict__ X, int64_t nnz, FV<R, NF>* As) {
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < E; k += (int64_t)gridDim.x * blockDim.x) {
         const int32_t e = emap[k];
         FV<R, NF> v;
 #pragma unroll
         for (int f = 0; f < NF; f++) v.v[f] = 0;
-        if (e >= 0) v = A[e];
+        if (e >= 0) v = e < nnz ? A[e] : X[e - nnz];
         As[k] = v;
     }
 }
@@ -44,6 +44,17 @@ __global__ void k_fill_tile_ell(int64_t E, const int32_t* __restrict__ emap, con
 constexpr int kHaloSlots = 1024;
 constexpr int kHaloSlotsMax = 16384;
 
+// A row's entries: the pattern's, or the given ones (ModRows).
+struct RowEntries {
+    const int32_t *col, *slot;  // slot null: entry e has slot first + e
+    int32_t first, n;
+};
+__device__ __forceinline__ RowEntries row_entries(const int32_t* rp, const int32_t* col, const ModRows& m, int64_t r) {
+    const int32_t k = m.of ? m.of[r] : -1;
+    if (k >= 0) return {m.col + m.off[k], m.slot + m.off[k], 0, m.off[k + 1] - m.off[k]};
+    return {col + rp[r], nullptr, rp[r], rp[r + 1] - rp[r]};
+}
+
 struct EllTotals {
     unsigned long long entries;
     int hmax, emax, overflow;
@@ -51,17 +62,18 @@ struct EllTotals {
 
 // Entries per slice (32 x its longest row) and per tile, one block per tile.
 __global__ void __launch_bounds__(kTileRows) k_slice_widths(const int32_t* __restrict__ rp,
-                                                            const int32_t* __restrict__ col, int64_t N, bool skip_diag,
-                                                            int32_t* width, EllTotals* tot) {
+                                                            const int32_t* __restrict__ col, ModRows mod, int64_t N,
+                                                            bool skip_diag, int32_t* width, EllTotals* tot) {
     __shared__ unsigned long long sum;
     if (threadIdx.x == 0) sum = 0;
     __syncthreads();
     const int64_t r = blockIdx.x * (int64_t)kTileRows + threadIdx.x;
     int32_t len = 0;
     if (r < N) {
-        len = rp[r + 1] - rp[r];
+        const RowEntries row = row_entries(rp, col, mod, r);
+        len = row.n;
         if (skip_diag)
-            for (int32_t e = rp[r]; e < rp[r + 1]; e++) len -= col[e] == r;
+            for (int32_t e = 0; e < row.n; e++) len -= row.col[e] == r;
     }
     const int32_t w = __reduce_max_sync(0xffffffffu, len);
     if ((threadIdx.x & 31) == 0) {
@@ -78,18 +90,16 @@ __global__ void __launch_bounds__(kTileRows) k_slice_widths(const int32_t* __res
 // The tile's columns outside it, as a hash set in shared memory (open
 // addressing, INT32_MAX empty).  Returns their number, or -1 past three
 // quarters of the slots.  Every thread of the block calls it.
-__device__ int halo_set(const int32_t* __restrict__ rp, const int32_t* __restrict__ col, int64_t N, int slots,
-                        int32_t* set) {
+__device__ int halo_set(const int32_t* __restrict__ rp, const int32_t* __restrict__ col, const ModRows& mod, int64_t N,
+                        int slots, int32_t* set) {
     __shared__ int count;
     const int64_t t0 = blockIdx.x * (int64_t)kTileRows, t1 = min(N, t0 + kTileRows);
     for (int i = threadIdx.x; i < slots; i += kTileRows) set[i] = INT32_MAX;
     if (threadIdx.x == 0) count = 0;
     __syncthreads();
     const int most = slots / 4 * 3;
-    const int32_t e1 = rp[t1];
-    for (int32_t e = rp[t0] + threadIdx.x; e < e1; e += kTileRows) {
-        const int32_t c = col[e];
-        if (c >= t0 && c < t1) continue;
+    auto add = [&](int32_t c) {
+        if (c >= t0 && c < t1) return;
         unsigned at = ((unsigned)c * 2654435761u >> 8) & (unsigned)(slots - 1);
         while (*(volatile int*)&count <= most) {
             const int32_t old = atomicCAS(&set[at], INT32_MAX, c);
@@ -97,16 +107,25 @@ __device__ int halo_set(const int32_t* __restrict__ rp, const int32_t* __restric
             if (old == INT32_MAX || old == c) break;
             at = (at + 1) & (unsigned)(slots - 1);
         }
+    };
+    // every entry of the pattern (a row given anew holds its old columns too),
+    // then the rows given anew
+    const int32_t e1 = rp[t1];
+    for (int32_t e = rp[t0] + threadIdx.x; e < e1; e += kTileRows) add(col[e]);
+    const int64_t r = t0 + threadIdx.x;
+    if (mod.of && r < t1 && mod.of[r] >= 0) {
+        const RowEntries row = row_entries(rp, col, mod, r);
+        for (int32_t e = 0; e < row.n; e++) add(row.col[e]);
     }
     __syncthreads();
     return count <= most ? count : -1;
 }
 
 __global__ void __launch_bounds__(kTileRows) k_halo_count(const int32_t* __restrict__ rp,
-                                                          const int32_t* __restrict__ col, int64_t N, int slots,
-                                                          int32_t* hcnt, EllTotals* tot) {
+                                                          const int32_t* __restrict__ col, ModRows mod, int64_t N,
+                                                          int slots, int32_t* hcnt, EllTotals* tot) {
     extern __shared__ int32_t set[];
-    const int n = halo_set(rp, col, N, slots, set);
+    const int n = halo_set(rp, col, mod, N, slots, set);
     if (threadIdx.x == 0) {
         hcnt[blockIdx.x] = max(n, 0);
         if (n < 0) atomicExch(&tot->overflow, 1);
@@ -116,12 +135,13 @@ __global__ void __launch_bounds__(kTileRows) k_halo_count(const int32_t* __restr
 
 // Halo lists (sorted), local columns, column pairs and slots of one tile.
 __global__ void __launch_bounds__(kTileRows) k_fill_pattern(const int32_t* __restrict__ rp,
-                                                            const int32_t* __restrict__ col, int64_t N, bool skip_diag,
-                                                            int slots, const int32_t* __restrict__ slice_off,
+                                                            const int32_t* __restrict__ col, ModRows mod, int64_t N,
+                                                            bool skip_diag, int slots,
+                                                            const int32_t* __restrict__ slice_off,
                                                             const int32_t* __restrict__ halo_off, int32_t* halo_col,
                                                             uint16_t* lcol, uint32_t* lcol2, int32_t* emap) {
     extern __shared__ int32_t set[];
-    const int n = halo_set(rp, col, N, slots, set);
+    const int n = halo_set(rp, col, mod, N, slots, set);
     for (int size = 2; size <= slots; size <<= 1)  // bitonic sort; the empty slots go last
         for (int stride = size >> 1; stride > 0; stride >>= 1) {
             for (int i = threadIdx.x; i < slots / 2; i += kTileRows) {
@@ -140,15 +160,16 @@ __global__ void __launch_bounds__(kTileRows) k_fill_pattern(const int32_t* __res
     const int lane = threadIdx.x & 31;
     const int64_t s = blockIdx.x * (int64_t)(kTileRows / 32) + (threadIdx.x >> 5);
     const int32_t sb = slice_off[s], w = (slice_off[s + 1] - sb) / 32;
-    int32_t e = r < N ? rp[r] : 0;
-    const int32_t e1 = r < N ? rp[r + 1] : 0;
+    RowEntries row{};
+    if (r < N) row = row_entries(rp, col, mod, r);
+    int32_t e = 0;
     uint32_t first = 0;
     for (int32_t k = 0; k < w; k++) {
-        if (skip_diag && e < e1 && col[e] == r) e++;
+        if (skip_diag && e < row.n && row.col[e] == r) e++;
         uint32_t lc = (uint32_t)threadIdx.x;  // padding: the row's own slot, value 0
         int32_t slot = -1;
-        if (e < e1) {
-            const int32_t c = col[e];
+        if (e < row.n) {
+            const int32_t c = row.col[e];
             if (c >= t0 && c < t0 + kTileRows) {
                 lc = (uint32_t)(c - t0);
             } else {
@@ -160,7 +181,8 @@ __global__ void __launch_bounds__(kTileRows) k_fill_pattern(const int32_t* __res
                 }
                 lc = (uint32_t)(kTileRows + lo);
             }
-            slot = e++;
+            slot = row.slot ? row.slot[e] : row.first + e;
+            e++;
         }
         const int32_t at = sb + 32 * k + lane;
         lcol[at] = (uint16_t)lc;
@@ -176,7 +198,8 @@ __global__ void __launch_bounds__(kTileRows) k_fill_pattern(const int32_t* __res
 }  // namespace
 
 bool build_tile_ell(const int32_t* rp, const int32_t* col, int64_t N, size_t fv_bytes, size_t smem_budget, TileEll& L,
-                    DeviceArena& keep, cudaStream_t st, bool skip_diag) {
+                    DeviceArena& keep, cudaStream_t st, bool skip_diag, const ModRows* given) {
+    const ModRows mod = given ? *given : ModRows{};
     L = TileEll{};
     if (N <= 0) return false;
     const int64_t ntiles = ceil_div(N, kTileRows), nslices = ntiles * (kTileRows / 32);
@@ -190,11 +213,11 @@ bool build_tile_ell(const int32_t* rp, const int32_t* col, int64_t N, size_t fv_
     int slots = kHaloSlots;
     for (;;) {
         FEA_CUDA_TRY(cudaMemsetAsync(tot, 0, sizeof(EllTotals), st));
-        k_slice_widths<<<(int)ntiles, kTileRows, 0, st>>>(rp, col, N, skip_diag, width, tot);
+        k_slice_widths<<<(int)ntiles, kTileRows, 0, st>>>(rp, col, mod, N, skip_diag, width, tot);
         FEA_CHECK_LAUNCH();
         if (slots > kHaloSlots)
             FEA_CUDA_TRY(cudaFuncSetAttribute(k_halo_count, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * slots));
-        k_halo_count<<<(int)ntiles, kTileRows, 4 * slots, st>>>(rp, col, N, slots, hcnt, tot);
+        k_halo_count<<<(int)ntiles, kTileRows, 4 * slots, st>>>(rp, col, mod, N, slots, hcnt, tot);
         FEA_CHECK_LAUNCH();
         FEA_CUDA_TRY(cudaMemcpyAsync(&h, tot, sizeof(h), cudaMemcpyDeviceToHost, st));
         FEA_CUDA_TRY(cudaStreamSynchronize(st));
@@ -221,7 +244,7 @@ bool build_tile_ell(const int32_t* rp, const int32_t* col, int64_t N, size_t fv_
     }
     if (slots > kHaloSlots)
         FEA_CUDA_TRY(cudaFuncSetAttribute(k_fill_pattern, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * slots));
-    k_fill_pattern<<<(int)ntiles, kTileRows, 4 * slots, st>>>(rp, col, N, skip_diag, slots, L.slice_off, L.halo_off,
+    k_fill_pattern<<<(int)ntiles, kTileRows, 4 * slots, st>>>(rp, col, mod, N, skip_diag, slots, L.slice_off, L.halo_off,
                                                               L.halo_col, L.lcol, L.lcol2, L.emap);
     FEA_CHECK_LAUNCH();
     L.ok = true;
@@ -229,15 +252,20 @@ bool build_tile_ell(const int32_t* rp, const int32_t* col, int64_t N, size_t fv_
 }
 
 template <typename R, int NF>
-void fill_tile_ell(const TileEll& L, const FV<R, NF>* A, FV<R, NF>* As, cudaStream_t st) {
+void fill_tile_ell(const TileEll& L, const FV<R, NF>* A, FV<R, NF>* As, cudaStream_t st, const FV<R, NF>* X,
+                   int64_t nnz) {
     if (!L.ok || L.E == 0) return;
-    k_fill_tile_ell<R, NF><<<launch_grid(L.E), kBlock, 0, st>>>(L.E, L.emap, A, As);
+    k_fill_tile_ell<R, NF><<<launch_grid(L.E), kBlock, 0, st>>>(L.E, L.emap, A, X, nnz, As);
     FEA_CHECK_LAUNCH();
 }
 
-template void fill_tile_ell<float, 1>(const TileEll&, const FV<float, 1>*, FV<float, 1>*, cudaStream_t);
-template void fill_tile_ell<float, 2>(const TileEll&, const FV<float, 2>*, FV<float, 2>*, cudaStream_t);
-template void fill_tile_ell<double, 1>(const TileEll&, const FV<double, 1>*, FV<double, 1>*, cudaStream_t);
-template void fill_tile_ell<double, 2>(const TileEll&, const FV<double, 2>*, FV<double, 2>*, cudaStream_t);
+template void fill_tile_ell<float, 1>(const TileEll&, const FV<float, 1>*, FV<float, 1>*, cudaStream_t, const FV<float, 1>*,
+                                      int64_t);
+template void fill_tile_ell<float, 2>(const TileEll&, const FV<float, 2>*, FV<float, 2>*, cudaStream_t, const FV<float, 2>*,
+                                      int64_t);
+template void fill_tile_ell<double, 1>(const TileEll&, const FV<double, 1>*, FV<double, 1>*, cudaStream_t, const FV<double, 1>*,
+                                      int64_t);
+template void fill_tile_ell<double, 2>(const TileEll&, const FV<double, 2>*, FV<double, 2>*, cudaStream_t, const FV<double, 2>*,
+                                      int64_t);
 
 }  // namespace fea
