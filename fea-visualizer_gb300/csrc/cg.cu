@@ -718,32 +718,6 @@ __global__ void __launch_bounds__(kBlock) k_cgcg_iter_stream(StepArgs<R, NF> a) 
 // block's partials; at the end, value k of the block's threads.
 
 
-// Totals of NV values over nb block partials p[k * stride + b]: warp k merges
-// value k (lane l takes b = l, l + 32, ... with 16 loads in flight, then a
-// shuffle tree), a fixed order; lane 0 of warp k leaves total k in sm[k].
-// Needs NV <= the block's warps; every thread calls it (no barrier inside).
-template <int NV, typename R>
-__device__ __forceinline__ void merge_partials_by_warp(const typename Acc<R>::Packed* p, int64_t stride, int nb,
-                                                       typename Acc<R>::Packed* sm) {
-    using P = typename Acc<R>::Packed;
-    constexpr int B = 16;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (w >= NV) return;
-    Acc<R> y;
-    for (int base = lane; base < nb; base += 32 * B) {
-        P v[B];
-#pragma unroll
-        for (int u = 0; u < B; u++)
-            if (base + 32 * u < nb) v[u] = __ldcg(&p[w * stride + base + 32 * u]);
-#pragma unroll
-        for (int u = 0; u < B; u++)
-            if (base + 32 * u < nb) y.merge(Acc<R>::unpack(v[u]));
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) y.shfl_add(o);
-    if (lane == 0) sm[w] = y.pack();
-}
-
 // Deferred finish at the start of a launch of buffer parity q (variants 12 to
 // 15): every block reads the state of parity q ^ 1 into st; when the previous
 // launch left an iteration pending, warp k merges value k of that launch's
@@ -2130,18 +2104,6 @@ __global__ void __launch_bounds__(kBlock) k_final_check(StepArgs<R, NF> a) {
 }
 
 // ---- stiff groups around a solve (stiff.cu) -------------------------------------------
-
-// The loop of a solve with stiff groups stops at an eighth of the tolerance;
-// the true-residual pass and its restart keep the tolerance itself.  The
-// diagonal iteration spends its last dozens of iterations on the stiff
-// groups while every other error component keeps falling; with the groups
-// solved exactly the loop ends sooner and leaves those components larger at
-// the same |r|.  Errors against FP64 after 10 Gray-Scott steps on the 1024 x
-// 1024 grid (u / v, four seeds): diagonal iteration 1.4 to 2.0e-6 / 3.4 to 3.9e-6
-// in 172 iterations a step; groups at a quarter 2.0e-6 / 3.1 to 4.2e-6 in 62,
-// at an eighth 1.6e-6 / 1.6 to 2.0e-6 in 68.  The square is a power of two, so
-// the threshold returns exactly.
-constexpr double kStiffTol2 = 0.015625;
 
 // Before the set-up product: r and z = D'^-1 r' of the groups' rows in the
 // basis, gamma = r.z with their share exchanged, and a zero start there (the

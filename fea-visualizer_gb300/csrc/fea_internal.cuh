@@ -98,6 +98,18 @@ struct StiffBasis {
     void* X = nullptr;     // [nx] values of A' (handle type, per field)
     void* dinv = nullptr;  // inverse diagonal of A'
 };
+// The loop of a solve with stiff groups stops at an eighth of the tolerance;
+// the true-residual pass and its restart keep the tolerance itself.  The
+// diagonal iteration spends its last dozens of iterations on the stiff
+// groups while every other error component keeps falling; with the groups
+// solved exactly the loop ends sooner and leaves those components larger at
+// the same |r|.  Errors against FP64 after 10 Gray-Scott steps on the 1024 x
+// 1024 grid (u / v, four seeds): diagonal iteration 1.4 to 2.0e-6 / 3.4 to 3.9e-6
+// in 172 iterations a step; groups at a quarter 2.0e-6 / 3.1 to 4.2e-6 in 62,
+// at an eighth 1.6e-6 / 1.6 to 2.0e-6 in 68.  The square is a power of two, so
+// the threshold returns exactly.
+constexpr double kStiffTol2 = 0.015625;
+
 // Groups of the pattern P's unknowns by its stiffness matrix K, four unknowns
 // each (-1 unused).
 std::vector<std::array<int32_t, 4>> find_stiff_groups(const Pattern& P, const double* K, cudaStream_t st);
@@ -177,6 +189,8 @@ struct RunState {
     long long steps_left, steps_done, total_iters;
     long long cg_launches;  // iteration kernels run (timing probes excluded)
     unsigned int flags;
+    int halt;             // resident launches: a launch of this call stopped early
+    unsigned int epoch;   // resident launches: the last exchange's number
     int last_iters[2];
     double last_rel[2];
     double tol;
@@ -291,6 +305,26 @@ void build_step_graph(StepGraph& g, const StepArgs<R, NF>& base, int kind, int l
 // (profiling mode: FEA_LAUNCH_MODE=stream).
 template <typename R, int NF>
 void run_steps_stream(const StepArgs<R, NF>& base, int kind, int lanes, LoopFlags* lf, cudaStream_t st);
+
+// ---- small and mid-size meshes: the whole step loop in one launch (resident.cu) --------
+struct ResidentPlan {
+    bool cluster = false;  // one thread block cluster; else a cooperative grid
+    int blocks = 0, T = 0, tpb = 0, passes = 0, us = 0;
+    size_t smem = 0;
+};
+// The launch shape of these arguments; false when the operator does not fit
+// the blocks' shared memory, the layout is out of the kernel's range or the
+// device cannot hold all blocks at once.
+template <typename R, int NF>
+bool plan_resident(const StepArgs<R, NF>& a, ResidentPlan& p);
+// Device memory through which a launch's blocks exchange (zeroed once).
+template <typename R, int NF>
+size_t resident_exchange_bytes(int64_t N);
+// nsteps steps of `kind` on the stream (Ks, Advs: tile-ELL copies of K and
+// Adv; where: the stiff groups' places by row, or null).
+template <typename R, int NF>
+void run_resident(const StepArgs<R, NF>& a, const ResidentPlan& p, const R* Ks, const R* Advs, const int32_t* where,
+                  void* exchange, int kind, int64_t nsteps, cudaStream_t st);
 
 // Timing and autotuning probe: one CG iteration kernel with the given window
 // size, after prepare_probe has masked every field (x and p are written back

@@ -197,9 +197,17 @@ struct fea_solver {
     TileEll ell_st;                 // the diagonal-free layout of A' = Q^T A Q
     void *S1s = nullptr, *S0s = nullptr, *S2s = nullptr;       // its copies of A1', A0', A2'
     StiffBasis B1, B0, B2;          // the bases of A1, A0, A2
+    bool stiff_stale[3] = {true, true, true};                  // A0', A1', A2' do not match their operators
     void* grp_x0 = nullptr;         // the groups' start values during a solve
     int* grp_in = nullptr;
-    bool diagonal_only = false;     // solves without the stiff groups (DiagonalOnly)
+    bool diagonal_only = false;     // solves without the stiff groups, on the step graph (DiagonalOnly)
+    void *Ks_ell = nullptr, *Advs_ell = nullptr;               // tile-ELL copies of K and Adv (resident launches)
+    bool resident = true;           // the step loop may run as one resident launch (no CG variant chosen)
+    struct {
+        int known = 0;              // 0: not asked, 1: fits, -1: does not
+        ResidentPlan plan;
+    } res[2][2];                    // by fields - 1 and stiff groups
+    void* exchange[2] = {nullptr, nullptr};  // by fields - 1: the blocks' exchange (first resident launch)
     uint8_t* adv_present = nullptr;
     Fields F;
     // loop state
@@ -235,12 +243,19 @@ size_t rsize(const fea_solver* s) { return s->precision == FEA_FP64 ? 8 : 4; }
 int ring_emax(const fea_solver* s) { return std::max(s->ell.emax, s->ell_st.emax); }
 int ring_hmax(const fea_solver* s) { return std::max(s->ell.hmax, s->ell_st.hmax); }
 
+// Tiles per SM up to which a mesh may run as a resident launch (resident.cu
+// has kernels for that many).
+constexpr int64_t kResidentTiles = 8;
+
 int64_t pad_tiles(int64_t n) { return ceil_div(n, kTileRows) * kTileRows; }
 
 void* ralloc(DeviceArena& ar, const fea_solver* s, int64_t n) {
     if (s->precision == FEA_FP64) return ar.alloc<double>(n);
     return ar.alloc<float>(n);
 }
+
+// n values of the handle's type past p.
+void* roffset(const fea_solver* s, void* p, int64_t n) { return (char*)p + rsize(s) * (size_t)n; }
 
 int step_kind(const fea_params& p) {
     switch (p.equation) {
@@ -281,11 +296,19 @@ void assemble(fea_solver* s) {
         round_copy<float>(s->M64, s->emap, s->P.nnz, (float*)s->Mc, s->stream);
         round_copy<float>(s->Adv64, s->emap, s->P.nnz, (float*)s->Advc, s->stream);
         fill_tile_ell<float, 1>(s->ell, (const FV<float, 1>*)s->Mc, (FV<float, 1>*)s->Ms_ell, s->stream);
+        if (s->Ks_ell) {
+            fill_tile_ell<float, 1>(s->ell, (const FV<float, 1>*)s->Kc, (FV<float, 1>*)s->Ks_ell, s->stream);
+            fill_tile_ell<float, 1>(s->ell, (const FV<float, 1>*)s->Advc, (FV<float, 1>*)s->Advs_ell, s->stream);
+        }
     } else {
         round_copy<double>(s->K64, s->emap, s->P.nnz, (double*)s->Kc, s->stream);
         round_copy<double>(s->M64, s->emap, s->P.nnz, (double*)s->Mc, s->stream);
         round_copy<double>(s->Adv64, s->emap, s->P.nnz, (double*)s->Advc, s->stream);
         fill_tile_ell<double, 1>(s->ell, (const FV<double, 1>*)s->Mc, (FV<double, 1>*)s->Ms_ell, s->stream);
+        if (s->Ks_ell) {
+            fill_tile_ell<double, 1>(s->ell, (const FV<double, 1>*)s->Kc, (FV<double, 1>*)s->Ks_ell, s->stream);
+            fill_tile_ell<double, 1>(s->ell, (const FV<double, 1>*)s->Advc, (FV<double, 1>*)s->Advs_ell, s->stream);
+        }
     }
     memcpy(s->cur_vel, s->prm.advdiff_velocity, sizeof(s->cur_vel));
     s->cur_vel_mode = s->prm.velocity_mode;
@@ -324,9 +347,9 @@ bool build_stiff_layout(fea_solver* s) {
                         &mod))
         return false;
     s->grp = G;
-    s->S1s = ralloc(s->mat_mem, s, s->ell_st.E);
-    s->S0s = ralloc(s->mat_mem, s, s->ell_st.E);
-    s->S2s = ralloc(s->mat_mem, s, 2 * s->ell_st.E);
+    s->S1s = ralloc(s->mat_mem, s, 4 * s->ell_st.E);
+    s->S0s = roffset(s, s->S1s, s->ell_st.E);
+    s->S2s = roffset(s, s->S0s, s->ell_st.E);
     const std::pair<StiffBasis*, int> bases[3] = {{&s->B1, 1}, {&s->B0, 1}, {&s->B2, 2}};
     for (const auto& b : bases) {
         b.first->Q = s->mat_mem.alloc<double>(16 * (int64_t)G.n * b.second);
@@ -356,6 +379,9 @@ void build_context(fea_solver* s) {
     s->Ms_ell = nullptr;
     s->grp = StiffGroups{};
     s->ell_st = TileEll{};
+    s->Ks_ell = s->Advs_ell = nullptr;
+    for (auto& r : s->res) r[0].known = r[1].known = 0;
+    s->exchange[0] = s->exchange[1] = nullptr;
     s->S1s = s->S0s = s->S2s = nullptr;
     s->B1 = s->B0 = s->B2 = StiffBasis{};
     s->F = Fields{};
@@ -375,14 +401,20 @@ void build_context(fea_solver* s) {
         const int32_t *rp = s->Pc.row_ptr, *col = s->Pc.col;
         build_tile_ell(rp, col, N, 2 * rsize(s), kEllSmemBudget, s->ell, s->mat_mem, st);
         if (s->ell.ok) {
-            s->S1 = ralloc(s->mat_mem, s, s->ell.E);
-            s->S0 = ralloc(s->mat_mem, s, s->ell.E);
-            s->S2 = ralloc(s->mat_mem, s, 2 * s->ell.E);
-            s->Ms_ell = ralloc(s->mat_mem, s, s->ell.E);
+            // one allocation per layout (E is a multiple of 32 entries)
+            const bool extra = ceil_div(N, kTileRows) <= kResidentTiles * (int64_t)num_sms();
+            s->S1 = ralloc(s->mat_mem, s, (extra ? 7 : 5) * s->ell.E);
+            s->S0 = roffset(s, s->S1, s->ell.E);
+            s->S2 = roffset(s, s->S0, s->ell.E);
+            s->Ms_ell = roffset(s, s->S2, 2 * s->ell.E);
+            if (extra) {
+                s->Ks_ell = roffset(s, s->Ms_ell, s->ell.E);
+                s->Advs_ell = roffset(s, s->Ks_ell, s->ell.E);
+            }
             if (build_tile_ell(rp, col, N, 2 * rsize(s), kEllSmemBudget, s->ell_od, s->mat_mem, st, true)) {
-                s->S1d = ralloc(s->mat_mem, s, s->ell_od.E);
-                s->S0d = ralloc(s->mat_mem, s, s->ell_od.E);
-                s->S2d = ralloc(s->mat_mem, s, 2 * s->ell_od.E);
+                s->S1d = ralloc(s->mat_mem, s, 4 * s->ell_od.E);
+                s->S0d = roffset(s, s->S1d, s->ell_od.E);
+                s->S2d = roffset(s, s->S0d, s->ell_od.E);
             }
             build_stiff_layout(s);
         }
@@ -460,10 +492,20 @@ void build_context(fea_solver* s) {
     FEA_CUDA_TRY(cudaStreamSynchronize(st));
 }
 
+// The FP32 wave on larger meshes: its velocity sums accelerations -c^2 M^-1 K u
+// whose FP32 rounding grows with the mesh (7e-5 of the velocity against FP64
+// on the 500 x 500 grid, whatever the solver), and a different order of the
+// sums moves it by a third of that.  Such handles keep the diagonal iteration
+// on the step graph, bit for bit.
+bool rounding_bound_wave(const fea_solver* s) {
+    return s->precision == FEA_FP32 && s->prm.equation == FEA_WAVE && s->N > 16384;
+}
+
 // Whether the current equation's solves run in the stiff groups' basis.
 // Implicit advection-diffusion does not: its operator is not symmetric, CG
 // may break down on it, and it keeps the iteration it had.
 bool stiff_solves(const fea_solver* s) {
+    if (rounding_bound_wave(s)) return false;
     const bool symmetric = s->prm.equation != FEA_ADVECTION_DIFFUSION || s->prm.advection_scheme == 1;
     return s->grp.n > 0 && is_ring_variant(s->lanes) && !s->diagonal_only && symmetric;
 }
@@ -477,6 +519,22 @@ void set_rws(StepArgs<R, NF>& a, FV<R, NF>* base, int64_t Np) {
         a.wb[k] = base + (2 + k) * Np;
         a.sb[k] = base + (4 + k) * Np;
     }
+}
+
+// The copy of A' = Q^T A Q in the stiff groups' basis, made when a solve first
+// wants it after the operator changed.
+template <typename R, int NF>
+void ensure_stiff(fea_solver* s, bool init_op) {
+    bool& stale = s->stiff_stale[NF == 2 ? 2 : init_op ? 0 : 1];
+    if (!stale) return;
+    const Fields& F = s->F;
+    const auto* A = (const FV<R, NF>*)(NF == 2 ? F.A2 : init_op ? F.A0 : F.A1);
+    const auto* dinv = (const FV<R, NF>*)(NF == 2 ? F.d2 : init_op ? F.d0 : F.d1);
+    const StiffBasis& B = NF == 2 ? s->B2 : init_op ? s->B0 : s->B1;
+    void* Ss = NF == 2 ? s->S2s : init_op ? s->S0s : s->S1s;
+    update_stiff_basis<R, NF>(s->grp, s->Pc, A, dinv, B, s->stream);
+    fill_tile_ell<R, NF>(s->ell_st, A, (FV<R, NF>*)Ss, s->stream, (const FV<R, NF>*)B.X, s->P.nnz);
+    stale = false;
 }
 
 template <typename R, int NF>
@@ -539,6 +597,7 @@ StepArgs<R, NF> make_args(fea_solver* s, bool init_op) {
             a.emax_od = od.emax;
         }
         if (stiff) {
+            ensure_stiff<R, NF>(s, init_op);
             const StiffBasis& B = NF == 2 ? s->B2 : init_op ? s->B0 : s->B1;
             a.dinv_it = (const FV<R, NF>*)B.dinv;
             a.ngrp = s->grp.n;
@@ -604,22 +663,12 @@ void upload_params(fea_solver* s) {
     FEA_CUDA_TRY(cudaStreamSynchronize(s->stream));
 }
 
-// The iteration's copies of an operator A: the diagonal-free layout Sd of A
-// itself and Ss of A' = Q^T A Q (with stiff groups).
-template <typename R, int NF>
-void fill_iterated(fea_solver* s, const void* A, const void* dinv, void* Sd, const StiffBasis& B, void* Ss) {
-    const auto* Av = (const FV<R, NF>*)A;
-    fill_tile_ell<R, NF>(s->ell_od, Av, (FV<R, NF>*)Sd, s->stream);
-    if (s->grp.n == 0) return;
-    update_stiff_basis<R, NF>(s->grp, s->Pc, Av, (const FV<R, NF>*)dinv, B, s->stream);
-    fill_tile_ell<R, NF>(s->ell_st, Av, (FV<R, NF>*)Ss, s->stream, (const FV<R, NF>*)B.X, s->P.nnz);
-}
-
 // Operator coefficients (the float parameters widened to double; the
 // operator is evaluated in FP64 and rounded once to the handle's type).
 template <typename R>
 void update_operator(fea_solver* s, int kind) {
     const fea_params& p = s->prm;
+    for (bool& stale : s->stiff_stale) stale = true;
     const double dt = time_step(p);
     if (kind == EQ_GS_REF || kind == EQ_GS_CONSISTENT) {
         OpCoef<2> c{};
@@ -628,7 +677,7 @@ void update_operator(fea_solver* s, int kind) {
         combine_operator<R, 2>(s->Pc, s->emap, s->M64, s->K64, s->Adv64, c, (FV<R, 2>*)s->F.A2, (FV<R, 2>*)s->F.d2,
                                s->stream);
         fill_tile_ell<R, 2>(s->ell, (const FV<R, 2>*)s->F.A2, (FV<R, 2>*)s->S2, s->stream);
-        fill_iterated<R, 2>(s, s->F.A2, s->F.d2, s->S2d, s->B2, s->S2s);
+        fill_tile_ell<R, 2>(s->ell_od, (const FV<R, 2>*)s->F.A2, (FV<R, 2>*)s->S2d, s->stream);
     } else {
         OpCoef<1> c{};
         c.f[0] = {dt, 0.0, 1.0, 0.0};
@@ -652,12 +701,12 @@ void update_operator(fea_solver* s, int kind) {
             combine_operator<R, 1>(s->Pc, s->emap, s->M64, s->K64, s->Adv64, m, (FV<R, 1>*)s->F.A0, (FV<R, 1>*)s->F.d0,
                                    s->stream);
             fill_tile_ell<R, 1>(s->ell, (const FV<R, 1>*)s->F.A0, (FV<R, 1>*)s->S0, s->stream);
-            fill_iterated<R, 1>(s, s->F.A0, s->F.d0, s->S0d, s->B0, s->S0s);
+            fill_tile_ell<R, 1>(s->ell_od, (const FV<R, 1>*)s->F.A0, (FV<R, 1>*)s->S0d, s->stream);
         }
         combine_operator<R, 1>(s->Pc, s->emap, s->M64, s->K64, s->Adv64, c, (FV<R, 1>*)s->F.A1, (FV<R, 1>*)s->F.d1,
                                s->stream);
         fill_tile_ell<R, 1>(s->ell, (const FV<R, 1>*)s->F.A1, (FV<R, 1>*)s->S1, s->stream);
-        fill_iterated<R, 1>(s, s->F.A1, s->F.d1, s->S1d, s->B1, s->S1s);
+        fill_tile_ell<R, 1>(s->ell_od, (const FV<R, 1>*)s->F.A1, (FV<R, 1>*)s->S1d, s->stream);
     }
 }
 
@@ -686,10 +735,10 @@ struct GuessOff {
     }
 };
 
-// Solves without the stiff groups while it lives: the FP32 Gray-Scott adjoint
-// returns FP64 parameter gradients, sums over FP32 fields whose last digits
-// follow the iteration's rounding, and keeps the diagonal iteration it was
-// validated with.
+// Solves without the stiff groups and on the step graph while it lives: the
+// FP32 Gray-Scott adjoint returns FP64 parameter gradients, sums over FP32
+// fields whose last digits follow the iteration's rounding, and keeps the
+// iteration it was validated with.
 struct DiagonalOnly {
     fea_solver* s;
     DiagonalOnly(fea_solver* h, bool on) : s(h) { s->diagonal_only = on; }
@@ -712,9 +761,37 @@ void ensure_layout(fea_solver* s, bool interleaved) {
     F.interleaved = interleaved;
 }
 
+// The resident launch's shape for these arguments, or null: the step graph.
+template <typename R, int NF>
+const ResidentPlan* resident_plan(fea_solver* s, const StepArgs<R, NF>& a) {
+    if (!s->resident || s->stream_mode || s->diagonal_only || !s->Ks_ell || rounding_bound_wave(s)) return nullptr;
+    auto& r = s->res[NF - 1][a.ngrp ? 1 : 0];
+    if (r.known == 0) r.known = plan_resident<R, NF>(a, r.plan) ? 1 : -1;
+    return r.known > 0 ? &r.plan : nullptr;
+}
+
+template <typename R, int NF>
+bool try_resident(fea_solver* s, const StepArgs<R, NF>& a, int kind, int64_t nsteps) {
+    const ResidentPlan* p = resident_plan<R, NF>(s, a);
+    if (!p) return false;
+    void*& ex = s->exchange[NF - 1];
+    if (!ex) {
+        const size_t n = resident_exchange_bytes<R, NF>(s->N);
+        ex = s->mat_mem.alloc<unsigned char>((int64_t)n);
+        FEA_CUDA_TRY(cudaMemsetAsync(ex, 0, n, s->stream));
+    }
+    run_resident<R, NF>(a, *p, (const R*)s->Ks_ell, (const R*)s->Advs_ell, s->grp.where, ex, kind, nsteps, s->stream);
+    return true;
+}
+
 template <typename R, int NF>
 void run_graph(fea_solver* s, StepGraph& g, int kind, bool init_op, int64_t nsteps) {
     const bool stream_mode = s->stream_mode;
+    {
+        StepArgs<R, NF> a = make_args<R, NF>(s, init_op);
+        set_x<R, NF>(s, a, kind);
+        if (try_resident<R, NF>(s, a, kind, nsteps)) return;
+    }
     if (!stream_mode && (!g.exec || g.kind != kind || g.lanes != s->lanes)) {
         StepArgs<R, NF> a = make_args<R, NF>(s, init_op);
         set_x<R, NF>(s, a, kind);
@@ -879,6 +956,7 @@ void ensure_operator(fea_solver* s, int kind) {
 // One solve A mu = lam with the graph g (built on first use).
 template <typename R, int NF>
 void run_given(fea_solver* s, StepGraph& g, const StepArgs<R, NF>& a) {
+    if (try_resident<R, NF>(s, a, EQ_GIVEN, 1)) return;
     long long ctl[2] = {1, 0};  // steps_left, steps_done
     FEA_CUDA_TRY(cudaMemcpyAsync(s->d_run, ctl, sizeof(ctl), cudaMemcpyHostToDevice, s->stream));
     FEA_CUDA_TRY(cudaMemsetAsync(&s->d_run->flags, 0, sizeof(unsigned int), s->stream));
@@ -970,7 +1048,7 @@ double adjoint_gs_core(fea_solver* s, const FV<R, 2>* x0, const FV<R, 2>* t, int
         throw Error{FEA_ERR_STATE};
     }
     const GuessOff guess_off(s);  // recomputed forward states must equal the forward sweep's
-    const DiagonalOnly diagonal(s, sizeof(R) == 4 && s->grp.n > 0);
+    const DiagonalOnly diagonal(s, sizeof(R) == 4);
     cudaStream_t st = s->stream;
     const int64_t N = s->N;
     const size_t xb = sizeof(FV<R, 2>) * (size_t)N;
@@ -1934,6 +2012,7 @@ int fea_set_cg_variant(fea_solver* s, int variant) {
     default: break;
     }
     s->lanes = variant;
+    s->resident = false;  // an explicit choice names the kernels of the step graph
     API_END
 }
 
