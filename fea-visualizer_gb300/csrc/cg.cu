@@ -2108,8 +2108,9 @@ __global__ void __launch_bounds__(kBlock) k_final_check(StepArgs<R, NF> a) {
 // Before the set-up product: r and z = D'^-1 r' of the groups' rows in the
 // basis, gamma = r.z with their share exchanged, and a zero start there (the
 // solve accumulates the correction Q y; the start values wait in grp_x0, so
-// they are rounded once).  One block; the groups are a few per thousand rows.
-constexpr int kStiffBlock = 512;
+// they are rounded once).  A thread per group, in many small blocks: one block
+// took 18 us for the 270 groups of the 1024 x 1024 grid, bound by its gathers.
+constexpr int kStiffBlock = 32;
 template <typename R, int NF>
 __global__ void __launch_bounds__(kStiffBlock) k_stiff_in(StepArgs<R, NF> a) {
     __shared__ double sm[32 * NF];
@@ -2122,7 +2123,7 @@ __global__ void __launch_bounds__(kStiffBlock) k_stiff_in(StepArgs<R, NF> a) {
     double corr[NF];
 #pragma unroll
     for (int f = 0; f < NF; f++) corr[f] = 0;
-    for (int g = threadIdx.x; g < a.ngrp; g += blockDim.x) {
+    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < a.ngrp; g += gridDim.x * blockDim.x) {
         FV<R, NF> r[4], z[4], d[4];
         int m[4];
 #pragma unroll
@@ -2159,18 +2160,19 @@ __global__ void __launch_bounds__(kStiffBlock) k_stiff_in(StepArgs<R, NF> a) {
             }
     }
     block_sum<NF>(corr, sm);
-    if (threadIdx.x == 0) {
+    double all[NF];
+    if (last_block_commit<NF>(corr, a.part, a.part_stride, a.tickets + 7, sm, all) && threadIdx.x == 0) {
 #pragma unroll
         for (int f = 0; f < NF; f++) {
             if (!cg->active[f]) continue;
             cg->thr[f] *= kStiffTol2;
             if constexpr (sizeof(R) == 4) {
-                const double g = (double)cg->ffrz[f][0] + (double)cg->ffrz[f][1] + corr[f];
+                const double g = (double)cg->ffrz[f][0] + (double)cg->ffrz[f][1] + all[f];
                 cg->rz[f] = g;
                 ff_store(cg->ffrz[f], ff_of(g));
                 ff_store(cg->ffthr[f], ff_of(cg->thr[f]));
             } else {
-                cg->rz[f] += corr[f];
+                cg->rz[f] += all[f];
             }
         }
         *a.grp_in = 1 + (cg->active[0] ? 1 : 0) + (NF > 1 && cg->active[NF - 1] ? 2 : 0);
@@ -2183,7 +2185,7 @@ template <typename R, int NF>
 __global__ void __launch_bounds__(kStiffBlock) k_stiff_out(StepArgs<R, NF> a) {
     const int in = *(volatile int*)a.grp_in;
     if (!in) return;
-    for (int g = threadIdx.x; g < a.ngrp; g += blockDim.x) {
+    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < a.ngrp; g += gridDim.x * blockDim.x) {
         FV<R, NF> y[4];
         int m[4];
 #pragma unroll
@@ -2207,7 +2209,8 @@ __global__ void __launch_bounds__(kStiffBlock) k_stiff_out(StepArgs<R, NF> a) {
         }
     }
     __syncthreads();  // every thread has read grp_in
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0 && atomicAdd(a.tickets + 7, 1u) == gridDim.x - 1) {  // so has every block
+        a.tickets[7] = 0;
         *a.grp_in = 0;
 #pragma unroll
         for (int f = 0; f < NF; f++)
@@ -2337,6 +2340,11 @@ struct RhsKernel {
     }
 };
 
+template <typename R, int NF>
+int stiff_grid(const StepArgs<R, NF>& a) {
+    return (int)std::min<int64_t>(max_grid_blocks(), ceil_div(a.ngrp, kStiffBlock));
+}
+
 // Arguments of a set-up product: with stiff groups the layout of A'.
 template <typename R, int NF>
 StepArgs<R, NF> init_args(StepArgs<R, NF> a) {
@@ -2431,11 +2439,11 @@ void build_graph_t(StepGraph& G, const StepArgs<R, NF>& base, LoopFlags* lf) {
     cudaGraph_t body1, body2;
     // one solve from the residual the pass before it left
     auto add_solve = [&](const StepArgs<R, NF>& la, cudaGraph_t* body) {
-        if (la.ngrp) s = add_kernel(step_body, s, k_stiff_in<R, NF>, 1, kStiffBlock, la);
+        if (la.ngrp) s = add_kernel(step_body, s, k_stiff_in<R, NF>, stiff_grid(la), kStiffBlock, la);
         s = add_kernel(step_body, s, K::init, g.spmv, kBlock, init_args(la), g.smem_init);
         s = add_while(step_body, s, la.cond, body);
         add_iterations<K>(*body, g.iter, la, g.smem_iter);
-        if (la.ngrp) s = add_kernel(step_body, s, k_stiff_out<R, NF>, 1, kStiffBlock, la);
+        if (la.ngrp) s = add_kernel(step_body, s, k_stiff_out<R, NF>, stiff_grid(la), kStiffBlock, la);
     };
     add_solve(L.a1, &body1);
     s = add_kernel(step_body, s, g.refine_k, g.refine, kBlock, L.a2, g.smem_refine);
@@ -2474,7 +2482,7 @@ void run_stream_t(const StepArgs<R, NF>& base, LoopFlags* lf, cudaStream_t st) {
                 FEA_CHECK_LAUNCH();
             }
             if (la->ngrp) {
-                k_stiff_in<R, NF><<<1, kStiffBlock, 0, st>>>(*la);
+                k_stiff_in<R, NF><<<stiff_grid(*la), kStiffBlock, 0, st>>>(*la);
                 FEA_CHECK_LAUNCH();
             }
             K::init<<<g.spmv, kBlock, g.smem_init, st>>>(init_args(*la));
@@ -2493,7 +2501,7 @@ void run_stream_t(const StepArgs<R, NF>& base, LoopFlags* lf, cudaStream_t st) {
                 }
             }
             if (la->ngrp) {
-                k_stiff_out<R, NF><<<1, kStiffBlock, 0, st>>>(*la);
+                k_stiff_out<R, NF><<<stiff_grid(*la), kStiffBlock, 0, st>>>(*la);
                 FEA_CHECK_LAUNCH();
             }
         }

@@ -154,6 +154,43 @@ struct Fields {
     void *xprev2 = nullptr, *xg2 = nullptr;  // Gray-Scott: previous state, extrapolated guess
 };
 
+// Device buffers a call needs, kept by the handle for the next call of the
+// same shape: the k-th request of a call gets the k-th buffer, made anew when
+// it is too small.  (Allocating and freeing took 50 us of a frame's normals
+// and 0.1 ms a buffer in the adjoints, and each free waits for the device.)
+struct Scratch {
+    Scratch() = default;
+    Scratch(const Scratch&) = delete;
+    Scratch& operator=(const Scratch&) = delete;
+    ~Scratch() { release(); }
+    std::vector<std::pair<void*, size_t>> bufs;
+    size_t next = 0;
+    void rewind() { next = 0; }
+    template <typename T>
+    T* alloc(int64_t count) {
+        const size_t need = (size_t)(count > 0 ? count : 1) * sizeof(T);
+        if (next == bufs.size()) bufs.emplace_back(nullptr, 0);
+        auto& b = bufs[next++];
+        if (b.second < need) {
+            cudaFree(b.first);
+            b = {nullptr, 0};
+            FEA_CUDA_TRY(cudaMalloc(&b.first, need));
+            b.second = need;
+        }
+        return static_cast<T*>(b.first);
+    }
+    int64_t bytes() const {
+        int64_t n = 0;
+        for (const auto& b : bufs) n += (int64_t)b.second;
+        return n;
+    }
+    void release() {
+        for (auto& b : bufs) cudaFree(b.first);
+        bufs.clear();
+        next = 0;
+    }
+};
+
 }  // namespace fea
 
 using namespace fea;
@@ -222,6 +259,11 @@ struct fea_solver {
     RunState* h_run = nullptr;  // pinned
     StepGraph graph, init_graph;
     StepGraph diag_graph;  // the step graph without the stiff groups
+    StepGraph given_graph[2];  // the adjoint's solve by fields - 1, and what it was built for
+    struct {
+        const void *x = nullptr, *rhs = nullptr, *op = nullptr;
+    } given_for[2];
+    Scratch scratch[3];  // adjoint sweeps, their entry points, smooth normals
     int lanes = 8;  // CG kernel variant: 0/1 tile-ELL (8/4 entries prefetched), 2/3 streamed (stages), 4/8/16 CSR window
     bool op_dirty = true;
     int op_kind = -1;
@@ -368,6 +410,7 @@ void build_context(fea_solver* s) {
     s->graph.destroy();
     s->init_graph.destroy();
     s->diag_graph.destroy();
+    for (auto& g : s->given_graph) g.destroy();
     s->mat_mem.release();
     s->P = Pattern{};
     s->Pc = Pattern{};
@@ -953,9 +996,11 @@ void ensure_operator(fea_solver* s, int kind) {
 // right-hand side; forward states are recomputed from checkpoints taken every
 // `ckpt` steps.
 
-// One solve A mu = lam with the graph g (built on first use).
+// One solve A mu = lam.  The graph is kept for the handle's next sweep; it
+// holds the addresses of mu, lam and the operator, and is rebuilt when one
+// of them (or the variant) is another.
 template <typename R, int NF>
-void run_given(fea_solver* s, StepGraph& g, const StepArgs<R, NF>& a) {
+void run_given(fea_solver* s, const StepArgs<R, NF>& a) {
     if (try_resident<R, NF>(s, a, EQ_GIVEN, 1)) return;
     long long ctl[2] = {1, 0};  // steps_left, steps_done
     FEA_CUDA_TRY(cudaMemcpyAsync(s->d_run, ctl, sizeof(ctl), cudaMemcpyHostToDevice, s->stream));
@@ -964,7 +1009,13 @@ void run_given(fea_solver* s, StepGraph& g, const StepArgs<R, NF>& a) {
         run_steps_stream<R, NF>(a, EQ_GIVEN, s->lanes, s->d_flags, s->stream);
         return;
     }
-    if (!g.exec) build_step_graph<R, NF>(g, a, EQ_GIVEN, s->lanes, s->d_flags);
+    StepGraph& g = s->given_graph[NF - 1];
+    auto& f = s->given_for[NF - 1];
+    if (!g.exec || g.lanes != s->lanes || f.x != a.x || f.rhs != a.rhs || f.op != a.As_od) {
+        FEA_CUDA_TRY(cudaStreamSynchronize(s->stream));  // the old graph may still run
+        build_step_graph<R, NF>(g, a, EQ_GIVEN, s->lanes, s->d_flags);
+        f = {a.x, a.rhs, a.As_od};
+    }
     FEA_CUDA_TRY(cudaGraphLaunch(g.exec, s->stream));
 }
 
@@ -984,7 +1035,8 @@ double adjoint_core(fea_solver* s, const R* u0, const R* t, int64_t nsteps, int6
     ckpt = std::min(ckpt, nsteps);
     const int64_t nck = ceil_div(nsteps, ckpt);
     ensure_layout<R>(s, false);
-    DeviceArena tmp;
+    Scratch& tmp = s->scratch[0];
+    tmp.rewind();
     R* ck = tmp.alloc<R>(nck * N);
     R* seg = tmp.alloc<R>((ckpt + 1) * N);
     R* mu = tmp.alloc<R>(pad_tiles(N));  // x of the solves: whole tiles
@@ -1005,7 +1057,6 @@ double adjoint_core(fea_solver* s, const R* u0, const R* t, int64_t nsteps, int6
         StepArgs<R, 1> a = make_args<R, 1>(s, false);
         a.x = (FV<R, 1>*)mu;
         a.rhs = (const FV<R, 1>*)lam_f;
-        StepGraph g;
         const double dt = time_step(s->prm), c = s->prm.advdiff_c, sign = s->prm.advection_sign;
         try {
             for (int64_t sg = nck - 1; sg >= 0; sg--) {
@@ -1016,18 +1067,15 @@ double adjoint_core(fea_solver* s, const R* u0, const R* t, int64_t nsteps, int6
                     FEA_CUDA_TRY(cudaMemcpyAsync(seg + (n - n0 + 1) * N, u, rb, d2d, st));
                 }
                 for (int64_t n = n1 - 1; n >= n0; n--) {
-                    run_given<R, 1>(s, g, a);  // mu = A^-1 lam, warm-started from the previous mu
+                    run_given<R, 1>(s, a);  // mu = A^-1 lam, warm-started from the previous mu
                     adjoint_grad_D<R>(s->Kloc, s->tri, s->idx_c, s->T, c, mu, seg + (n - n0 + 1) * N, gD, st);
                     adjoint_lambda<R>(s->Pc, (const R*)s->Mc, (const R*)s->Advc, dt, sign, mu, lam_f, st);
                 }
             }
         } catch (...) {
             cudaStreamSynchronize(st);
-            g.destroy();
             throw;
         }
-        FEA_CUDA_TRY(cudaStreamSynchronize(st));
-        g.destroy();
     }
     FEA_CUDA_TRY(cudaMemcpyAsync(u, uN, rb, d2d, st));
     double h = 0;
@@ -1056,7 +1104,8 @@ double adjoint_gs_core(fea_solver* s, const FV<R, 2>* x0, const FV<R, 2>* t, int
     ckpt = std::min(ckpt, nsteps);
     const int64_t nck = ceil_div(nsteps, ckpt);
     ensure_layout<R>(s, true);  // the forward steps update the operator to the current parameters
-    DeviceArena tmp;
+    Scratch& tmp = s->scratch[0];
+    tmp.rewind();
     FV<R, 2>* ck = tmp.alloc<FV<R, 2>>(nck * N);
     FV<R, 2>* seg = tmp.alloc<FV<R, 2>>((ckpt + 1) * N);
     FV<R, 2>* mu = tmp.alloc<FV<R, 2>>(pad_tiles(N));  // x of the solves: whole tiles
@@ -1076,7 +1125,6 @@ double adjoint_gs_core(fea_solver* s, const FV<R, 2>* x0, const FV<R, 2>* t, int
         StepArgs<R, 2> a = make_args<R, 2>(s, false);
         a.x = mu;
         a.rhs = lam;
-        StepGraph gr;
         const fea_params& p = s->prm;
         const double dt = p.rd_time_step, F = p.rd_feed_rate, kr = p.rd_kill_rate;
         try {
@@ -1089,7 +1137,7 @@ double adjoint_gs_core(fea_solver* s, const FV<R, 2>* x0, const FV<R, 2>* t, int
                     FEA_CUDA_TRY(cudaMemcpyAsync(seg + (n - n0 + 1) * N, x, xb, d2d, st));
                 }
                 for (int64_t n = n1 - 1; n >= n0; n--) {
-                    run_given<R, 2>(s, gr, a);  // mu = A^-1 lam (both fields), warm-started
+                    run_given<R, 2>(s, a);  // mu = A^-1 lam (both fields), warm-started
                     adjoint_gs_step<R>(s->Pc, (const R*)s->Mc, (const R*)s->Kc, mu, seg + (n - n0) * N,
                                        seg + (n - n0 + 1) * N, dt, F, kr, lam, s->d_part, max_grid_blocks(),
                                        s->d_tickets + 6, g, st);
@@ -1097,11 +1145,8 @@ double adjoint_gs_core(fea_solver* s, const FV<R, 2>* x0, const FV<R, 2>* t, int
             }
         } catch (...) {
             cudaStreamSynchronize(st);
-            gr.destroy();
             throw;
         }
-        FEA_CUDA_TRY(cudaStreamSynchronize(st));
-        gr.destroy();
     }
     FEA_CUDA_TRY(cudaMemcpyAsync(x, xN, xb, d2d, st));
     double h = 0;
@@ -1116,7 +1161,8 @@ void adjoint_gs_host(fea_solver* s, const float* u0, const float* v0, const floa
                      int64_t nsteps, int64_t ckpt, double* loss, float* gu, float* gv, double* gparams) {
     cudaStream_t st = s->stream;
     const int64_t N = s->N, V = s->V;
-    DeviceArena tmp;
+    Scratch& tmp = s->scratch[1];
+    tmp.rewind();
     FV<R, 2>* x0 = tmp.alloc<FV<R, 2>>(N);
     FV<R, 2>* t = tmp.alloc<FV<R, 2>>(N);
     FV<R, 2>* lam = tmp.alloc<FV<R, 2>>(N);
@@ -1153,7 +1199,8 @@ void adjoint_gs_device(fea_solver* s, const void* u0, const void* v0, const void
                        int64_t nsteps, int64_t ckpt, double* loss, void* gu, void* gv, double* gparams) {
     cudaStream_t st = s->stream;
     const int64_t N = s->N;
-    DeviceArena tmp;
+    Scratch& tmp = s->scratch[1];
+    tmp.rewind();
     FV<R, 2>* x0 = tmp.alloc<FV<R, 2>>(N);
     FV<R, 2>* t = tmp.alloc<FV<R, 2>>(N);
     FV<R, 2>* lam = tmp.alloc<FV<R, 2>>(N);
@@ -1188,7 +1235,8 @@ void adjoint_host(fea_solver* s, const float* u0, const float* target, int64_t n
                   float* grad_u0, float* grad_D) {
     cudaStream_t st = s->stream;
     const int64_t N = s->N, V = s->V, T = s->T;
-    DeviceArena tmp;
+    Scratch& tmp = s->scratch[1];
+    tmp.rewind();
     R* u0s = tmp.alloc<R>(N);
     R* ts = tmp.alloc<R>(N);
     R* lam = tmp.alloc<R>(N);
@@ -1222,7 +1270,8 @@ void adjoint_device(fea_solver* s, const void* u0, const void* target, int64_t n
                     void* grad_u0, void* grad_D) {
     cudaStream_t st = s->stream;
     const int64_t N = s->N, T = s->T;
-    DeviceArena tmp;
+    Scratch& tmp = s->scratch[1];
+    tmp.rewind();
     R* u0s = tmp.alloc<R>(N);
     R* ts = tmp.alloc<R>(N);
     R* lam = tmp.alloc<R>(N);
@@ -1296,14 +1345,11 @@ void ensure_vertex_triangles(fea_solver* s) {
     build_vertex_triangles(s->tri, s->T, s->V, s->vt_ptr, s->vt_tri, s->stream);
 }
 
-// nrm and out: device float[3V]
-void smooth_normals_dev(fea_solver* s, const float* nrm, float e, float* out) {
+// nrm and out: device float[3V]; face: float[3T] scratch
+void smooth_normals_dev(fea_solver* s, const float* nrm, float e, float* face, float* out) {
     ensure_vertex_triangles(s);
     stage_node_values(s);
-    DeviceArena tmp;
-    float* face = tmp.alloc<float>(3 * s->T);
     smooth_normals(s->xyz, s->tri, s->T, s->V, s->vt_ptr, s->vt_tri, nrm, s->d_nodes, e, face, out, s->stream);
-    FEA_CUDA_TRY(cudaStreamSynchronize(s->stream));
 }
 
 struct PlyGeometry {
@@ -1572,9 +1618,11 @@ int fea_destroy(fea_solver* s) {
     s->graph.destroy();
     s->init_graph.destroy();
     s->diag_graph.destroy();
+    for (auto& g : s->given_graph) g.destroy();
     s->mat_mem.release();
     s->run_mem.release();
     s->mesh_mem.release();
+    for (Scratch& k : s->scratch) k.release();
     if (s->h_run) cudaFreeHost(s->h_run);
     if (s->stream) cudaStreamDestroy(s->stream);
     delete s;
@@ -1685,11 +1733,13 @@ int fea_smooth_normals(fea_solver* s, const float* normals, float vertex_extrusi
     API_BEGIN
     check_handle(s);
     if (!normals || !out) return fail(FEA_ERR_INVALID_ARGUMENT, "null normals or output");
-    DeviceArena tmp;
+    Scratch& tmp = s->scratch[2];
+    tmp.rewind();
+    float* face = tmp.alloc<float>(3 * s->T);
     float* nrm = tmp.alloc<float>(3 * s->V);
     float* res = tmp.alloc<float>(3 * s->V);
     FEA_CUDA_TRY(cudaMemcpyAsync(nrm, normals, sizeof(float) * 3 * s->V, cudaMemcpyHostToDevice, s->stream));
-    smooth_normals_dev(s, nrm, vertex_extrusion, res);
+    smooth_normals_dev(s, nrm, vertex_extrusion, face, res);
     FEA_CUDA_TRY(cudaMemcpyAsync(out, res, sizeof(float) * 3 * s->V, cudaMemcpyDeviceToHost, s->stream));
     FEA_CUDA_TRY(cudaStreamSynchronize(s->stream));
     API_END
@@ -1699,7 +1749,10 @@ int fea_smooth_normals_device(fea_solver* s, const float* normals, float vertex_
     API_BEGIN
     check_handle(s);
     if (!normals || !out) return fail(FEA_ERR_INVALID_ARGUMENT, "null normals or output");
-    smooth_normals_dev(s, normals, vertex_extrusion, out);
+    Scratch& tmp = s->scratch[2];
+    tmp.rewind();
+    smooth_normals_dev(s, normals, vertex_extrusion, tmp.alloc<float>(3 * s->T), out);
+    FEA_CUDA_TRY(cudaStreamSynchronize(s->stream));
     API_END
 }
 
@@ -1915,6 +1968,7 @@ int fea_get_info(fea_solver* s, fea_info* out) {
     out->boundary_condition = s->bc;
     out->rows_per_warp_lanes = s->lanes;
     out->device_bytes = s->mesh_mem.bytes + s->mat_mem.bytes + s->run_mem.bytes;
+    for (const Scratch& k : s->scratch) out->device_bytes += k.bytes();
     API_END
 }
 
