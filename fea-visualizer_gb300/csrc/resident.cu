@@ -25,7 +25,8 @@
 // else): 1,750 in a cluster of 16 against 3,430 through the L2; 128 blocks
 // 5,120 through block 0 against 8,740 with every block reading every partial
 // (the polls of all blocks meet on the same lines) and about 7,300 for a
-// counter barrier and a second read.
+// counter barrier and a second read.  In this kernel the every-block form took
+// 11.1 ms against 6.3 (Gray-Scott, 251 x 251 grid, 124 blocks, 20 steps).
 //
 // Per iteration a block publishes only w' = A u' of its rows.  A halo slot's
 // thread keeps its own copy of the halo row's r and s and advances them from
@@ -402,6 +403,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
         ph ^= 1;
         return __syncthreads_or(*(volatile int*)&dead) == 0;  // the same answer in every thread
     };
+    auto x_epoch = [&]() FEA_INLINE { return ++epoch != 0 ? epoch : ++epoch; };  // (0 has a meaning, below)
     auto total = [&](int k) FEA_INLINE { return Acc<R>::unpack(reinterpret_cast<typename Acc<R>::Packed*>(tot)[k]); };
 
     const int kind = ra.kind;
@@ -610,7 +612,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
         }
         // ---- x_n to the history, the start to x -------------------------------------
         const bool send_x = gs && step == 0;  // the next step wants x_(n-1) at its halos
-        if (send_x) xep[1] = ++epoch;
+        if (send_x) xep[1] = x_epoch();
 #pragma unroll
         for (int q = 0; q < kP; q++) {
             cx[q] = cp[q] = V{};
@@ -927,7 +929,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
                 __syncthreads();
             }
             // x to global memory and to the halos; zero right-hand sides give x = 0
-            xep[xb] = ++epoch;
+            xep[xb] = x_epoch();
 #pragma unroll
             for (int q = 0; q < kP; q++) {
                 if (rowq[q] < 0) continue;

@@ -5,6 +5,8 @@ the two agree to the rounding of their sums.  Sizes at the edges of the launch
 shapes: one tile, two tiles in one block, a cluster's first and last sizes,
 the cooperative grid's first, and several tiles per block.
 """
+import threading
+
 import numpy as np
 import pytest
 
@@ -124,3 +126,37 @@ def test_iteration_limit_and_zero_field(fea):
     assert rel_l2(b[0][0], a[0][0]) < 1e-6
     a, b = _both(fea, xyz, tri, 1, 0, _params(fea, "gs0", 0, False), 2, (u, 0 * u))
     assert rel_l2(b[0][0], a[0][0]) < 1e-5 and np.all(b[0][1] == 0) and np.all(a[0][1] == 0)
+
+
+def test_handles_on_several_threads(fea):
+    """Handles stepped at once from threads of their own (one block, a cluster, two
+    device-wide grids and the step graph) give what each gives alone."""
+    shapes = [(10, 10, 0, "heat"), (64, 60, 0, "gs1"), (128, 129, 1, "heat"), (251, 251, 0, "gs1"), (251, 251, 0, "heat")]
+    handles, fields = [], []
+    for nx, ny, prec, eq in shapes:
+        xyz, tri = mg.cylinder(nx, ny)
+        handles.append(fea.CUDASolver(xyz, tri, boundary_condition=1, precision=prec, params=_params(fea, eq, prec, False)))
+        w = np.random.default_rng(nx).uniform(size=(2, len(xyz)))
+        fields.append(np.stack([1 - 0.5 * w[0], 0.25 * w[1]]).astype(np.float32))
+    handles[-1].set_cg_variant(14)
+
+    def work(i, out):
+        s = handles[i]
+        s.clear_values()
+        s.set_fields(*fields[i])
+        for _ in range(5):
+            s.advance_time(4)
+        st = s.status()
+        out[i] = (s.get_fields(), st.flags, st.steps_done)
+
+    alone, together = {}, {}
+    for i in range(len(shapes)):
+        work(i, alone)
+    threads = [threading.Thread(target=work, args=(i, together)) for i in range(len(shapes))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for i in range(len(shapes)):
+        assert together[i][1:] == alone[i][1:] == (0, 4)
+        assert all(np.array_equal(a, b) for a, b in zip(together[i][0], alone[i][0]))
