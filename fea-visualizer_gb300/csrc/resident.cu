@@ -49,11 +49,12 @@ constexpr long long kWaitClocks = 6000000000ll;  // about 3 s of waiting at most
 constexpr int64_t kResidentSteps = 256;          // steps of one launch at most
 constexpr int kMaxBlocks = 160;                  // slots per value of the partials' buffers
 constexpr int kClusterBlocks = 16;               // blocks of a cluster launch (above 8: opt-in)
-// Tiles per block up to which a mesh runs as one cluster.  Heat on a grid, one
-// cluster against a cooperative grid of one-tile blocks: FP32 27 tiles 816
-// against 856 us (228 iterations), 38 tiles (three a block) 1397 against 1200
-// (308); FP64, bound by the SMs' FP64 rate, 14 tiles even, 20 tiles (two a block)
-// 2865 against 2373 (413).
+// Tiles per block up to which a mesh runs as one cluster.  Heat on a grid, 6
+// steps, one cluster against a cooperative grid of one-tile blocks: FP32 16
+// tiles 1,233 against 1,381 us, 27 tiles (two a block) 1,155 against 1,397;
+// three a block lost (38 tiles 1,397 against 1,200).  FP64, bound by the SMs'
+// FP64 rate: 16 tiles 2,650 against 3,060 us, two a block lost (20 tiles 2,865
+// against 2,373, 413 iterations).
 template <typename R>
 constexpr int kClusterTiles = sizeof(R) == 4 ? 2 : 1;
 
@@ -1109,13 +1110,11 @@ bool plan_resident(const StepArgs<R, NF>& a, ResidentPlan& p) {
     const int64_t ntiles = ceil_div(a.N, kTileRows);
     const int64_t most = std::min(num_sms(), kMaxBlocks);
     // up to two tiles in one block (no exchange at all), then one cluster, then
-    // the whole device
+    // the whole device, as few tiles a block as it has SMs for (two a block on
+    // half the blocks: heat, 142 tiles, 3,351 against 3,135 us, Gray-Scott 2,673
+    // against 2,449)
     p.cluster = ntiles > 2 && ntiles <= kClusterBlocks * kClusterTiles<R>;
     int64_t T = ntiles <= 2 ? ntiles : ceil_div(ntiles, p.cluster ? (int64_t)kClusterBlocks : most);
-    // FP32: from 64 blocks on, half as many with two tiles each meet sooner than
-    // they take longer (heat, 146 tiles, 630 iterations: 2.66 against 2.95 ms; 64
-    // tiles 1.43 against 1.46 ms)
-    if (!p.cluster && sizeof(R) == 4 && ntiles > 64) T = std::max<int64_t>(T, 2);
     const auto al = [](size_t x) { return (x + 15) & ~(size_t)15; };
     p.T = (int)T;
     p.blocks = (int)ceil_div(ntiles, T);
