@@ -1,5 +1,6 @@
 // cg.cu -- the per-step hot path: fused right-hand side, Jacobi-preconditioned
-// CG and the step loop, all inside one CUDA graph.
+// CG and the step loop, all inside one CUDA graph (small and mid-size meshes
+// run the same recurrences in one kernel, resident.cu).
 //
 // Reference semantics: CPUSolver::advance_time (CPUSolver.cpp:64-146) solves
 // A x = b with Eigen::ConjugateGradient<.., Lower|Upper> and its diagonal

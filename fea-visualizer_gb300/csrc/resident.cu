@@ -1074,6 +1074,10 @@ ResidentFn<R, NF> resident_kernel(int passes) {
         if (passes <= 3) return k_resident<R, NF, 3>;
         if (passes <= 4) return k_resident<R, NF, 4>;
     }
+    // (a sixth pass spills too much: heat, 640 x 640 grid, 48.2 ms against the
+    // graph's 39.2; five passes, 590 x 590, 28.5 against 33.0)
+    if constexpr (sizeof(R) * NF == 4)
+        if (passes <= 5) return k_resident<R, NF, 5>;
     return nullptr;
 }
 

@@ -287,7 +287,7 @@ int ring_hmax(const fea_solver* s) { return std::max(s->ell.hmax, s->ell_st.hmax
 
 // Tiles per SM up to which a mesh may run as a resident launch (resident.cu
 // has kernels for that many).
-constexpr int64_t kResidentTiles = 8;
+int64_t resident_tiles(const fea_solver* s) { return s->precision == FEA_FP32 ? 10 : 8; }
 
 int64_t pad_tiles(int64_t n) { return ceil_div(n, kTileRows) * kTileRows; }
 
@@ -445,7 +445,7 @@ void build_context(fea_solver* s) {
         build_tile_ell(rp, col, N, 2 * rsize(s), kEllSmemBudget, s->ell, s->mat_mem, st);
         if (s->ell.ok) {
             // one allocation per layout (E is a multiple of 32 entries)
-            const bool extra = ceil_div(N, kTileRows) <= kResidentTiles * (int64_t)num_sms();
+            const bool extra = ceil_div(N, kTileRows) <= resident_tiles(s) * (int64_t)num_sms();
             s->S1 = ralloc(s->mat_mem, s, (extra ? 7 : 5) * s->ell.E);
             s->S0 = roffset(s, s->S1, s->ell.E);
             s->S2 = roffset(s, s->S0, s->ell.E);

@@ -144,7 +144,8 @@ typedef struct {
     int64_t steps_done;          /* steps completed by the last fea_advance_time */
     int64_t total_iterations;    /* CG iterations summed over all solves */
     int64_t cg_launches;         /* CG iteration kernels launched, including the copies
-                                    that close an unrolled loop pass without iterating */
+                                    that close an unrolled loop pass without iterating
+                                    (steps run as one kernel count their iterations) */
 } fea_status;
 
 typedef struct fea_solver fea_solver;
@@ -211,7 +212,8 @@ int fea_set_fields_device(fea_solver* s, const void* u, const void* v);
 int fea_get_fields_device(fea_solver* s, void* u, void* v);
 
 /* Solver::advance_time (CPUSolver.cpp:64-146) nsteps times.  The whole step
- * loop runs as one CUDA graph launch; stepping stops early once
+ * loop runs on the device, as one CUDA graph launch or, on small and mid-size
+ * meshes, as one kernel per 256 steps; stepping stops early once
  * FEA_STATUS_BLOWUP or FEA_STATUS_NONFINITE is raised (the application pauses
  * there, Application.cpp:532-538).  Asynchronous: returns after the launch. */
 int fea_advance_time(fea_solver* s, int64_t nsteps);
@@ -258,7 +260,8 @@ int fea_get_idx_map(fea_solver* s, int32_t* idx_map, uint8_t* on_boundary);
  * one CG iteration of each candidate on this mesh and keeps the fastest
  * (fea_info.rows_per_warp_lanes); the fields are left unchanged. */
 int fea_autotune(fea_solver* s);
-/* Select a variant explicitly (FEA_ERR_INVALID_ARGUMENT for another value,
+/* Select a variant explicitly; the handle then runs the step graph on any
+ * mesh (FEA_ERR_INVALID_ARGUMENT for another value,
  * FEA_ERR_UNSUPPORTED for the tile-ELL variants when the layout, or for the
  * streamed and ring variants the shared memory of their stages, is
  * unavailable on this mesh). */

@@ -69,6 +69,13 @@ def test_sizes_match_step_graph(fea, nx, ny, prec, eq):
     assert abs(b[1] - a[1]) <= 6 + a[1] // 50  # a solve may stop an iteration earlier or later
 
 
+# three, four and five passes of a block's thread groups (on 152 SMs)
+@pytest.mark.parametrize("nx,ny,prec,eq", [(400, 480, 0, "gs1"), (400, 480, 1, "heat"), (500, 480, 0, "gs1"),
+                                           (500, 480, 1, "heat"), (500, 480, 0, "heat"), (600, 600, 0, "heat")])
+def test_many_tiles_per_block(fea, nx, ny, prec, eq):
+    test_sizes_match_step_graph(fea, nx, ny, prec, eq)
+
+
 @pytest.mark.parametrize("eq", ["heat", "advdiff", "explicit", "wave", "newmark", "gs0", "gs1"])
 @pytest.mark.parametrize("n", [40, 150])  # 7 tiles (cluster) and 88 (grid)
 @pytest.mark.parametrize("bc", [0, 1])
