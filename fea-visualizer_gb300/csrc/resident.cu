@@ -831,11 +831,11 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
                         break;
                     }
                     // the CG scalars (finish_cgcg), a lane of warp 0 per field
+                    Inv g{}, den{};
                     if (threadIdx.x < 32) {
                         const Acc<R> ag = total(sf), ad = total(NF + sf), rr = total(2 * NF + sf);
                         it++;
                         int state = 0;  // 0: iterates, 1: converged, 2: breakdown
-                        Inv g{}, den{};
                         R al = 0, be = 0;
                         if constexpr (sizeof(R) == 4) {
                             const FF r2 = ff_norm(rr);
@@ -876,8 +876,9 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
                         }
                         if (threadIdx.x == 0) ctl.any = cont;
                         sact = on && cont;
-                        __syncthreads();
-                        // off the other warps' path: the next iteration's reciprocals
+                    }
+                    __syncthreads();
+                    if (threadIdx.x < 32) {  // off the other warps' path: the next iteration's reciprocals
                         if constexpr (sizeof(R) == 4) {
                             rgam = ff_rcp(g);
                             ralp = ff_mul(den, rgam);
@@ -885,8 +886,6 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
                             rgam = 1 / g;
                             ralp = den * rgam;
                         }
-                    } else {
-                        __syncthreads();
                     }
                     more = ctl.any;
                 }
