@@ -234,25 +234,18 @@ __device__ __forceinline__ void warp_scatter_sums(const A (&in)[N], typename A::
     if ((lane & (32 / W - 1)) == 0 && slot < N) out[slot] = v[0].pack();
 }
 
+__device__ __forceinline__ FF from_lane(const FF& x, int lane) {
+    FF y;
+    y.hi = __shfl_sync(0xffffffffu, x.hi, lane);
+    y.lo = __shfl_sync(0xffffffffu, x.lo, lane);
+    return y;
+}
+
 // Lane 0's packed accumulator in every lane.
 __device__ __forceinline__ float2 lane0(float2 v) {
     return make_float2(__shfl_sync(0xffffffffu, v.x, 0), __shfl_sync(0xffffffffu, v.y, 0));
 }
 __device__ __forceinline__ double lane0(double v) { return __shfl_sync(0xffffffffu, v, 0); }
-
-// a / b with one reciprocal: its product with a, corrected by the exact
-// remainder (about 46 bits).  Half the dependent operations of ff_div, which
-// divides twice; one warp computes the scalars while the others wait.
-__device__ __forceinline__ FF ff_div_fast(const FF& a, const FF& b) {
-    const float rc = __frcp_rn(b.hi), q = __fmul_rn(a.hi, rc);
-    const float r = __fadd_rn(__fmaf_rn(-q, b.hi, a.hi), __fmaf_rn(-q, b.lo, a.lo));
-    return ff_quick(q, __fmul_rn(r, rc));
-}
-__device__ __forceinline__ FF ff_rcp(const FF& x) {
-    FF one;
-    one.hi = 1.f;
-    return ff_div_fast(one, x);
-}
 
 // Everything a launch adds to the step's arguments.
 template <typename R>
@@ -272,7 +265,6 @@ template <typename R, int NF, int kP>
 __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, ResidentArgs<R> ra) {
     using V = FV<R, NF>;
     constexpr int NV = 3 * NF;
-    using Inv = std::conditional_t<sizeof(R) == 4, FF, double>;
     extern __shared__ __align__(16) unsigned char dyn[];
     __shared__ double red[kResThreads / 32][8];  // packed accumulators (8 bytes of either type)
     __shared__ double tot[8];
@@ -751,21 +743,9 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
                     }
                 }
                 __syncthreads();
-                // warp 0, lane f: field f's threshold, 1 / gamma and 1 / alpha (the next
-                // iteration's scalars then hold one division), iteration count
-                const int sf = min((int)(threadIdx.x & 31), NF - 1);
-                Inv rgam{}, ralp{}, thr{};
+                const int sf = (int)(threadIdx.x % NF);  // warp 0: the field of a lane's scalars
                 int it = st.iter, sact = ctl.act[sf];
                 const int most = st.max_iter;
-                if constexpr (sizeof(R) == 4) {
-                    rgam = ff_rcp(Acc<float>::unpack(make_float2(st.ffrz[sf][0], st.ffrz[sf][1])));
-                    ralp = ff_rcp(Acc<float>::unpack(make_float2(st.ffalpha[sf][0], st.ffalpha[sf][1])));
-                    thr = Acc<float>::unpack(make_float2(st.ffthr[sf][0], st.ffthr[sf][1]));
-                } else {
-                    rgam = 1 / st.rz[sf];
-                    ralp = 1 / st.alpha[sf];
-                    thr = st.thr[sf];
-                }
                 int more = ctl.any;
                 for (int k = 0; more; k++) {
                     // the halos' w, wanted after the rows' updates
@@ -830,35 +810,49 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
                         failed = true;
                         break;
                     }
-                    // the CG scalars (finish_cgcg), a lane of warp 0 per field
-                    Inv g{}, den{};
+                    // The CG scalars as finish_cgcg computes them, in warp 0: beta = g / gamma,
+                    // den = delta - beta (g / alpha), alpha = g / den.  The first two divisions
+                    // run side by side, lanes below NF taking g / gamma and the next NF
+                    // g / alpha.  They are divisions: a product with a kept reciprocal rounds
+                    // once more and overflows where gamma is below 2^-128.
                     if (threadIdx.x < 32) {
                         const Acc<R> ag = total(sf), ad = total(NF + sf), rr = total(2 * NF + sf);
                         it++;
                         int state = 0;  // 0: iterates, 1: converged, 2: breakdown
                         R al = 0, be = 0;
+                        volatile CgState* const sv = &st;  // gamma and alpha live there: fewer registers
+                        const bool second = threadIdx.x >= NF;
                         if constexpr (sizeof(R) == 4) {
-                            const FF r2 = ff_norm(rr);
-                            g = ff_norm(ag);
-                            const FF beta = ff_mul(g, rgam);
-                            den = ff_sub(ff_norm(ad), ff_mul(ff_mul(beta, g), ralp));
-                            const FF alpha = ff_div_fast(g, den);
+                            const FF r2 = ff_norm(rr), g = ff_norm(ag);
+                            const FF quot = ff_div(g, ff_load(second ? sv->ffalpha[sf] : sv->ffrz[sf]));
+                            const FF beta = from_lane(quot, sf), ga = from_lane(quot, NF + sf);
+                            const FF den = ff_sub(ff_norm(ad), ff_mul(beta, ga));
+                            const FF alpha = ff_div(g, den);
                             al = alpha.rounded();
                             be = beta.rounded();
                             state = !isfinite(r2.hi) ? 2
-                                    : ff_less(r2, thr) ? 1
+                                    : ff_less(r2, ff_load(sv->ffthr[sf])) ? 1
                                     : !(den.hi > 0.f) || !isfinite(alpha.hi) || !isfinite(beta.hi) ? 2
                                                                                                     : 0;
+                            if (threadIdx.x < NF) {
+                                ff_store(sv->ffrz[sf], g);
+                                ff_store(sv->ffalpha[sf], alpha);
+                            }
                         } else {
-                            g = ag.s;
-                            const double beta = g * rgam;
-                            den = ad.s - beta * g * ralp;
-                            al = g / den;
+                            const double g = ag.s, quot = g / (second ? sv->alpha[sf] : sv->rz[sf]);
+                            const double beta = __shfl_sync(0xffffffffu, quot, sf),
+                                         ga = __shfl_sync(0xffffffffu, quot, NF + sf);
+                            const double den = ad.s - beta * ga, alpha = g / den;
+                            al = alpha;
                             be = beta;
                             state = !isfinite(rr.s) ? 2
-                                    : rr.s < thr    ? 1
-                                    : !(den > 0.0) || !isfinite(al) || !isfinite(be) ? 2
-                                                                                    : 0;
+                                    : rr.s < sv->thr[sf] ? 1
+                                    : !(den > 0.0) || !isfinite(alpha) || !isfinite(beta) ? 2
+                                                                                          : 0;
+                            if (threadIdx.x < NF) {
+                                sv->rz[sf] = g;
+                                sv->alpha[sf] = alpha;
+                            }
                         }
                         const bool on = sact && state == 0;
                         const bool cont = __any_sync(0xffffffffu, on) && it < most;
@@ -878,15 +872,6 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
                         sact = on && cont;
                     }
                     __syncthreads();
-                    if (threadIdx.x < 32) {  // off the other warps' path: the next iteration's reciprocals
-                        if constexpr (sizeof(R) == 4) {
-                            rgam = ff_rcp(g);
-                            ralp = ff_mul(den, rgam);
-                        } else {
-                            rgam = 1 / g;
-                            ralp = den * rgam;
-                        }
-                    }
                     more = ctl.any;
                 }
                 if (failed) break;
