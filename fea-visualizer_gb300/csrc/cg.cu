@@ -2166,7 +2166,7 @@ __global__ void __launch_bounds__(kStiffBlock) k_stiff_in(StepArgs<R, NF> a) {
 #pragma unroll
         for (int f = 0; f < NF; f++) {
             if (!cg->active[f]) continue;
-            cg->thr[f] *= kStiffTol2;
+            cg->thr[f] = stiff_threshold<R>(cg->thr[f]);
             if constexpr (sizeof(R) == 4) {
                 const double g = (double)cg->ffrz[f][0] + (double)cg->ffrz[f][1] + all[f];
                 cg->rz[f] = g;
@@ -2215,7 +2215,7 @@ __global__ void __launch_bounds__(kStiffBlock) k_stiff_out(StepArgs<R, NF> a) {
         *a.grp_in = 0;
 #pragma unroll
         for (int f = 0; f < NF; f++)
-            if ((in - 1) >> f & 1) a.cg->thr[f] /= kStiffTol2;
+            if ((in - 1) >> f & 1) a.cg->thr[f] = solve_threshold<R>(a.run->tol, a.cg->bb[f]);
     }
 }
 

@@ -706,17 +706,29 @@ __device__ __forceinline__ void set_gamma(volatile S* s, int f, const Acc<R>& g)
     if constexpr (sizeof(R) == 4) ff_store(s->ffrz[f], ff_norm(g));
 }
 
-// CG scalars of a solve's start, per field: |b|^2, the threshold tol^2 |b|^2
-// (at least the smallest normal number of R), |r|^2 and gamma = r.z.  The
-// FP32 solver keeps float-float copies of gamma and the threshold for its
-// iterations.  Returns whether the field iterates.
+// |r|^2 below which a solve has converged: tol^2 |b|^2, at least the smallest
+// normal number of R; and below which its loop in the stiff groups' basis stops
+// (kStiffTol2), with the same floor: neither asks for sums of denormals.
+template <typename R>
+constexpr double kSmallestNormal = sizeof(R) == 4 ? 1.1754943508222875e-38 : 2.2250738585072014e-308;
+template <typename R>
+__device__ __forceinline__ double solve_threshold(double tol, double bb) {
+    const double thr = tol * tol * bb;
+    return thr < kSmallestNormal<R> ? kSmallestNormal<R> : thr;
+}
+template <typename R>
+__device__ __forceinline__ double stiff_threshold(double thr) {
+    const double t = thr * kStiffTol2;
+    return t < kSmallestNormal<R> ? kSmallestNormal<R> : t;
+}
+
+// CG scalars of a solve's start, per field: |b|^2, its threshold, |r|^2 and
+// gamma = r.z.  The FP32 solver keeps float-float copies of gamma and the
+// threshold for its iterations.  Returns whether the field iterates.
 template <typename R, typename S>
 __device__ __forceinline__ int start_solve(volatile S* s, int f, int stop, double tol, const Acc<R>& bb_a,
                                            const Acc<R>& rr_a, const Acc<R>& rz_a) {
-    const double tiny = sizeof(R) == 4 ? 1.1754943508222875e-38 : 2.2250738585072014e-308;
-    const double bb = bb_a.value(), rr = rr_a.value();
-    double thr = tol * tol * bb;
-    thr = thr < tiny ? tiny : thr;
+    const double bb = bb_a.value(), rr = rr_a.value(), thr = solve_threshold<R>(tol, bb);
     s->bb[f] = bb;
     s->thr[f] = thr;
     s->rr[f] = rr;

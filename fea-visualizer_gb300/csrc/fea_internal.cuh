@@ -106,8 +106,7 @@ struct StiffBasis {
 // the same |r|.  Errors against FP64 after 10 Gray-Scott steps on the 1024 x
 // 1024 grid (u / v, four seeds): diagonal iteration 1.4 to 2.0e-6 / 3.4 to 3.9e-6
 // in 172 iterations a step; groups at a quarter 2.0e-6 / 3.1 to 4.2e-6 in 62,
-// at an eighth 1.6e-6 / 1.6 to 2.0e-6 in 68.  The square is a power of two, so
-// the threshold returns exactly.
+// at an eighth 1.6e-6 / 1.6 to 2.0e-6 in 68.
 constexpr double kStiffTol2 = 0.015625;
 
 // Groups of the pattern P's unknowns by its stiffness matrix K, four unknowns

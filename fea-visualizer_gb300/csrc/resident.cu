@@ -671,7 +671,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
 #pragma unroll
                     for (int f = 0; f < NF; f++) {
                         if (!st.active[f]) continue;
-                        st.thr[f] *= kStiffTol2;
+                        st.thr[f] = stiff_threshold<R>(st.thr[f]);
                         if constexpr (sizeof(R) == 4) {
                             const double g = (double)st.ffrz[f][0] + (double)st.ffrz[f][1] + tot[f];
                             st.rz[f] = g;
@@ -909,7 +909,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
                     if (threadIdx.x == 0)
 #pragma unroll
                         for (int f = 0; f < NF; f++)
-                            if (was[f]) st.thr[f] /= kStiffTol2;
+                            if (was[f]) st.thr[f] = solve_threshold<R>(run->tol, st.bb[f]);
                 }
                 __syncthreads();
             }
