@@ -752,7 +752,7 @@ __device__ __forceinline__ bool deferred_head(const StepArgs<R, NF>& a, int q, C
             int act[NF];
 #pragma unroll
             for (int f = 0; f < NF; f++) act[f] = st.active[f];
-            finish_cgcg<R, NF>((volatile CgState*)&st, &sflags, act, tot);
+            finish_cgcg<R, NF>((volatile CgState*)&st, &sflags, act, tot, a.ngrp ? &a.run->tol : nullptr);
             st.pending = 0;
         }
         __syncthreads();

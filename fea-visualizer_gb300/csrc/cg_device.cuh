@@ -775,8 +775,11 @@ __device__ void finish_spmv(volatile S* cg, unsigned int* flags, const int (&act
 // gamma' = r.u, delta' = w.u and r.r per field.  Returns whether another
 // iteration runs.  The FP32 solver does this in float-float arithmetic and
 // stores |r|^2 as a double only when a field stops iterating.
+// tol: the caller's tolerance where the loop's threshold is a stricter one (null:
+// it is the threshold); the limit is judged by it.
 template <typename R, int NF, typename S>
-__device__ bool finish_cgcg(volatile S* cg, unsigned int* flags, const int (&act)[NF], const Acc<R>* tot) {
+__device__ bool finish_cgcg(volatile S* cg, unsigned int* flags, const int (&act)[NF], const Acc<R>* tot,
+                            const double* tol = nullptr) {
     const int it = cg->iter + 1;
     cg->iter = it;
     int any = 0;
@@ -835,14 +838,17 @@ __device__ bool finish_cgcg(volatile S* cg, unsigned int* flags, const int (&act
     }
     const bool cont = any && it < cg->max_iter;
     if (any && !cont) {
-        atomicOr(flags, FEA_STATUS_NOT_CONVERGED);
+        int missed = 0;
 #pragma unroll
         for (int f = 0; f < NF; f++)
             if (cg->active[f]) {
-                if constexpr (sizeof(R) == 4) cg->rr[f] = tot[2 * NF + f].value();
+                const double rr = tot[2 * NF + f].value();
+                if constexpr (sizeof(R) == 4) cg->rr[f] = rr;
                 cg->active[f] = 0;
                 cg->iters[f] = it;
+                missed |= !tol || !(rr < *tol * *tol * cg->bb[f]);
             }
+        if (missed) atomicOr(flags, FEA_STATUS_NOT_CONVERGED);
     }
     return cont;
 }

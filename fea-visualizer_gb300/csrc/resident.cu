@@ -864,8 +864,10 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
                                 st.active[sf] = 0;
                                 st.iters[sf] = it;
                                 st.rr[sf] = rr.value();
-                                if (state != 1)
-                                    atomicOr(&sflags, state == 2 ? FEA_STATUS_BREAKDOWN : FEA_STATUS_NOT_CONVERGED);
+                                // (the limit is judged by the caller's tolerance, not the groups' stricter stop)
+                                if (state == 2) atomicOr(&sflags, FEA_STATUS_BREAKDOWN);
+                                else if (state == 0 && !(stiff && rr.value() < run->tol * run->tol * st.bb[sf]))
+                                    atomicOr(&sflags, FEA_STATUS_NOT_CONVERGED);
                             }
                         }
                         if (threadIdx.x == 0) ctl.any = cont;
