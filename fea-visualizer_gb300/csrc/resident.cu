@@ -5,10 +5,10 @@
 // and a step's other passes and loop nodes another 50 to 120 us.  Here one
 // launch runs every step: each block owns a run of 256-row tiles, keeps their
 // diagonal-free tile-ELL operator (tile_ell.cu) in shared memory and its rows'
-// CG vectors in registers for the whole launch.  The recurrences, the sums'
-// precision and the CG scalars are those of the ring kernels: every block
-// merges all blocks' partials in one fixed order and so computes the same
-// scalars.
+// CG vectors in registers for the whole launch.  The recurrences and the sums'
+// precision are those of the ring kernels; of the CG scalars, beta g / alpha is
+// taken as beta (g / alpha), with as many roundings.  Every block merges all
+// blocks' partials in one fixed order and so computes the same scalars.
 //
 // What the blocks exchange carries its own arrival flag: every 4-byte word
 // travels in an 8-byte store beside a 4-byte epoch, and the reader polls the
@@ -704,9 +704,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
                 __syncthreads();
                 uint32_t wep2 = ++epoch;
                 {
-                    R dw[NF];
-#pragma unroll
-                    for (int f = 0; f < NF; f++) dw[f] = 0;
+                    Acc<R> acc[NF];  // exact products, as in the ring kernels' set-up
 #pragma unroll
                     for (int q = 0; q < kP; q++) {
                         if (rowq[q] < 0) continue;
@@ -714,11 +712,8 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
                         put(ra.wl[0], rowq[q], cw[q], wep2);
                         const V z = ub_of(q)[t];
 #pragma unroll
-                        for (int f = 0; f < NF; f++) dw[f] = fmar(cw[q].v[f], z.v[f], dw[f]);
+                        for (int f = 0; f < NF; f++) acc[f].add_prod(z.v[f], cw[q].v[f]);
                     }
-                    Acc<R> acc[NF];
-#pragma unroll
-                    for (int f = 0; f < NF; f++) acc[f].add(dw[f]);
                     if (!reduce(acc)) {
                         failed = true;
                         break;
