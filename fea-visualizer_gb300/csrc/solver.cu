@@ -280,10 +280,14 @@ namespace {
 
 size_t rsize(const fea_solver* s) { return s->precision == FEA_FP64 ? 8 : 4; }
 
-// The widest tile and halo of the ring kernels' layouts: the once-per-step
-// passes stream the full layout, the iteration one without the diagonal.
-int ring_emax(const fea_solver* s) { return std::max(s->ell.emax, s->ell_st.emax); }
-int ring_hmax(const fea_solver* s) { return std::max(s->ell.hmax, s->ell_st.hmax); }
+// Whether a ring variant's iteration fits a block's shared memory on the layout
+// L at `stages` stages (both field counts do when two fields do).
+bool ring_fits(const fea_solver* s, const TileEll& L, int stages) {
+    const size_t need = s->precision == FEA_FP64 ? ring_smem_bytes<double, 2>(L.emax, L.hmax, stages)
+                                                 : ring_smem_bytes<float, 2>(L.emax, L.hmax, stages);
+    return need <= kStreamSmemLimit;
+}
+int ring_stages(int lanes) { return lanes == 14 ? 3 : lanes == 15 ? 4 : 0; }
 
 // Tiles per SM up to which a mesh may run as a resident launch (resident.cu
 // has kernels for that many).
@@ -386,8 +390,11 @@ bool build_stiff_layout(fea_solver* s) {
     ModRows mod;
     if (groups.empty() || !plan_stiff_rows(groups, s->Pc, s->pos, G, mod, s->mat_mem, st) ||
         !build_tile_ell(s->Pc.row_ptr, s->Pc.col, N, 2 * rsize(s), kEllSmemBudget, s->ell_st, s->mat_mem, st, true,
-                        &mod))
+                        &mod) ||
+        !ring_fits(s, s->ell_st, 3)) {  // the groups' rows are longer: the kernel stays, they go
+        s->ell_st = TileEll{};
         return false;
+    }
     s->grp = G;
     s->S1s = ralloc(s->mat_mem, s, 4 * s->ell_st.E);
     s->S0s = roffset(s, s->S1s, s->ell_st.E);
@@ -468,12 +475,8 @@ void build_context(fea_solver* s) {
         // default variant: direct row loads with the operator ring (14) when
         // its stages fit, else the streamed deferred-finish kernel with as
         // many stages as fit, else the tile-ELL kernel, else windowed CSR
-        const int remax = ring_emax(s);
-        const int rhmax = ring_hmax(s);
-        const size_t ring = s->precision == FEA_FP64 ? ring_smem_bytes<double, 2>(remax, rhmax, 3)
-                                                     : ring_smem_bytes<float, 2>(remax, rhmax, 3);
         s->lanes = !s->ell.ok ? 8
-                   : ring <= kStreamSmemLimit ? 14
+                   : ring_fits(s, s->ell, 3)  ? 14
                    : s->stream_stages >= 3    ? 11
                    : s->stream_stages >= 2    ? 10
                                               : 0;
@@ -550,7 +553,8 @@ bool rounding_bound_wave(const fea_solver* s) {
 bool stiff_solves(const fea_solver* s) {
     if (rounding_bound_wave(s)) return false;
     const bool symmetric = s->prm.equation != FEA_ADVECTION_DIFFUSION || s->prm.advection_scheme == 1;
-    return s->grp.n > 0 && is_ring_variant(s->lanes) && !s->diagonal_only && symmetric;
+    return s->grp.n > 0 && is_ring_variant(s->lanes) && ring_fits(s, s->ell_st, ring_stages(s->lanes)) &&
+           !s->diagonal_only && symmetric;
 }
 
 // r, w and s of the Chronopoulos-Gear iteration, two buffers each, carved
@@ -2007,17 +2011,21 @@ int fea_get_idx_map(fea_solver* s, int32_t* idx_map, uint8_t* on_boundary) {
 static int variant_check(const fea_solver* s, int l) {
     const bool csr = l == 4 || l == 8 || l == 16;
     const int stages = (l == 2 || l == 6 || l == 10) ? 2 : (l == 3 || l == 7 || l == 11) ? 3 : 0;
-    const int ring = l == 14 ? 3 : l == 15 ? 4 : 0;
+    const int ring = ring_stages(l);
     if (!csr && l != 0 && l != 1 && l != 13 && stages == 0 && ring == 0) return FEA_ERR_INVALID_ARGUMENT;
     if (!csr && !s->ell.ok) return FEA_ERR_UNSUPPORTED;
     if (s->stream_stages < stages) return FEA_ERR_UNSUPPORTED;
-    if (ring) {
-        const size_t need = s->precision == FEA_FP64 ? ring_smem_bytes<double, 2>(ring_emax(s), ring_hmax(s), ring)
-                                                     : ring_smem_bytes<float, 2>(ring_emax(s), ring_hmax(s), ring);
-        if (need > kStreamSmemLimit) return FEA_ERR_UNSUPPORTED;
-    }
+    if (ring && !ring_fits(s, s->ell, ring)) return FEA_ERR_UNSUPPORTED;
     return FEA_OK;
 }
+
+// The handle's variant while it lives.
+struct VariantFor {
+    fea_solver* s;
+    int was;
+    VariantFor(fea_solver* h, int l) : s(h), was(h->lanes) { s->lanes = l; }
+    ~VariantFor() { s->lanes = was; }
+};
 
 int fea_autotune(fea_solver* s) {
     API_BEGIN
@@ -2034,6 +2042,7 @@ int fea_autotune(fea_solver* s) {
     int best_l = s->lanes;
     for (int l : cand) {
         if (variant_check(s, l)) continue;
+        const VariantFor probed(s, l);  // a variant's arguments are its own (which layout, deferred finish)
         probe_any(s, kind, l, true);
         for (int rep = 0; rep < 23; rep++) {
             if (rep == 3) FEA_CUDA_TRY(cudaEventRecord(e0, s->stream));
