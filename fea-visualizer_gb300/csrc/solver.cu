@@ -547,14 +547,18 @@ bool rounding_bound_wave(const fea_solver* s) {
     return s->precision == FEA_FP32 && s->prm.equation == FEA_WAVE && s->N > 16384;
 }
 
+// Whether variant l iterates in the basis of the handle's stiff groups.
+bool stiff_variant(const fea_solver* s, int l) {
+    return s->grp.n > 0 && is_ring_variant(l) && ring_fits(s, s->ell_st, ring_stages(l));
+}
+
 // Whether the current equation's solves run in the stiff groups' basis.
 // Implicit advection-diffusion does not: its operator is not symmetric, CG
 // may break down on it, and it keeps the iteration it had.
 bool stiff_solves(const fea_solver* s) {
     if (rounding_bound_wave(s)) return false;
     const bool symmetric = s->prm.equation != FEA_ADVECTION_DIFFUSION || s->prm.advection_scheme == 1;
-    return s->grp.n > 0 && is_ring_variant(s->lanes) && ring_fits(s, s->ell_st, ring_stages(s->lanes)) &&
-           !s->diagonal_only && symmetric;
+    return stiff_variant(s, s->lanes) && !s->diagonal_only && symmetric;
 }
 
 // r, w and s of the Chronopoulos-Gear iteration, two buffers each, carved
@@ -2041,7 +2045,10 @@ int fea_autotune(fea_solver* s) {
     float best = 1e30f;
     int best_l = s->lanes;
     for (int l : cand) {
-        if (variant_check(s, l)) continue;
+        // on a mesh with stiff groups only the variants that use them: the others take
+        // more iterations (170 against 68 a step on the 1024 x 1024 Gray-Scott grid),
+        // which the time of one does not show
+        if (variant_check(s, l) || (s->grp.n > 0 && !stiff_variant(s, l))) continue;
         const VariantFor probed(s, l);  // a variant's arguments are its own (which layout, deferred finish)
         probe_any(s, kind, l, true);
         for (int rep = 0; rep < 23; rep++) {

@@ -258,7 +258,10 @@ int fea_get_idx_map(fea_solver* s, int32_t* idx_map, uint8_t* on_boundary);
  * its ring does not fit in shared memory, 10 when only two streamed stages
  * fit, 0 when none do, 8 without the tile-ELL layout).  fea_autotune times
  * one CG iteration of each candidate on this mesh and keeps the fastest
- * (fea_info.rows_per_warp_lanes); the fields are left unchanged. */
+ * (fea_info.rows_per_warp_lanes); the fields are left unchanged.  On a mesh
+ * with stiff groups (nearly degenerate triangles) the candidates are the
+ * variants that iterate in the groups' basis, of 14 and 15: the others take
+ * more iterations. */
 int fea_autotune(fea_solver* s);
 /* Select a variant explicitly; the handle then runs the step graph on any
  * mesh (FEA_ERR_INVALID_ARGUMENT for another value,

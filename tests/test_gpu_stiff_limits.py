@@ -1,4 +1,4 @@
-"""Stiff groups against the caller's settings: the iteration limit,
+"""Stiff groups against the caller's settings: the iteration limit, autotuning,
 refinement modes and the extrapolated start, in the resident launch and on the
 step graph's own kernels."""
 import numpy as np
@@ -68,6 +68,24 @@ def test_limit_two_fields(fea, variant):
         if st.total_iterations < limit:
             break
     assert flags[0] == 4 and flags[-1] == 0
+
+
+@pytest.mark.parametrize("n", [68, 130, 300])
+@pytest.mark.parametrize("prec", [0, 1])
+def test_autotune_keeps_the_groups(fea, n, prec):
+    """The variant autotuning leaves behind takes no more iterations than the default."""
+    xyz, tri = flattened(n, 0.02, CELLS)
+    its = []
+    for tune in (False, True):
+        p = _heat(fea, prec, cg_tolerance=1e-10 if prec else 1e-6)
+        s = fea.CUDASolver(xyz, tri, boundary_condition=fea.NEUMANN, precision=prec, params=p)
+        if tune:
+            s.autotune()
+        s.set_values(_noise(len(xyz)))
+        s.advance_time(2)
+        assert s.status().flags == 0
+        its.append(s.status().total_iterations)
+    assert its[1] <= its[0] + 2, (its, s.info.rows_per_warp_lanes)
 
 
 @pytest.mark.parametrize("variant", [None, 14, 15])
