@@ -274,6 +274,10 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
         R alpha[NF], beta[NF];
         int act[NF], any;
     } ctl;
+    __shared__ struct {  // the last completed step's solves
+        int iters[NF];
+        double rr[NF], bb[NF];
+    } last;
     __shared__ unsigned int sflags;
     __shared__ int dead, sstop;
     const int grp = threadIdx.x >> 8, t = threadIdx.x & 255, lane = t & 31, w8 = t >> 5;
@@ -1000,6 +1004,13 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
         }
         done++;
         iters += st.iter;
+        if (threadIdx.x == 0)  // the next step's start rewrites them, and it may stop there
+#pragma unroll
+            for (int f = 0; f < NF; f++) {
+                last.iters[f] = st.iters[f];
+                last.rr[f] = st.rr[f];
+                last.bb[f] = st.bb[f];
+            }
     }
     if (ra.cluster) cluster_barrier();  // no block leaves while another may write into it
     if (dead) {
@@ -1032,8 +1043,8 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
         run->cg_launches += iters;
         if (done > 0) {
             for (int f = 0; f < NF; f++) {
-                run->last_iters[f] = st.iters[f];
-                run->last_rel[f] = st.bb[f] > 0.0 ? sqrt(st.rr[f] / st.bb[f]) : 0.0;
+                run->last_iters[f] = last.iters[f];
+                run->last_rel[f] = last.bb[f] > 0.0 ? sqrt(last.rr[f] / last.bb[f]) : 0.0;
             }
             if (gs && a.xprev) run->prev_valid = 1;
         }
