@@ -2,6 +2,7 @@
 #pragma once
 
 #include <array>
+#include <cstddef>
 #include <vector>
 
 #include "fea_common.cuh"
@@ -187,8 +188,10 @@ struct CgState {
 struct RunState {
     long long steps_left, steps_done, total_iters;
     long long cg_launches;  // iteration kernels run (timing probes excluded)
+    // kRunFlagBytes from here on are cleared as a run starts
     unsigned int flags;
     int halt;             // resident launches: a launch of this call stopped early
+    long long lost;       // resident launches: steps of the call an expired wait left undone in some block
     unsigned int epoch;   // resident launches: the last exchange's number
     int last_iters[2];
     double last_rel[2];
@@ -198,6 +201,8 @@ struct RunState {
     int guess;       // Gray-Scott: 1 starts each step's CG from 2 x_n - x_(n-1)
     int prev_valid;  // x_(n-1) of the extrapolation is the previous step's state
 };
+
+constexpr size_t kRunFlagBytes = offsetof(RunState, epoch) - offsetof(RunState, flags);
 
 // Everything a step-loop kernel needs, passed by value.
 template <typename R, int NF>

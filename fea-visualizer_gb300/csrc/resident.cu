@@ -37,6 +37,7 @@
 // cooperative launch.  Every wait is bounded; on expiry the launch raises
 // FEA_STATUS_BREAKDOWN and leaves.
 #include <algorithm>
+#include <cstdlib>
 #include <type_traits>
 
 #include "cg_device.cuh"
@@ -45,7 +46,7 @@ namespace fea {
 namespace {
 
 constexpr int kResThreads = 512;  // two tiles of 256 rows at a time; 128 registers a thread
-constexpr long long kWaitClocks = 6000000000ll;  // about 3 s of waiting at most
+constexpr long long kWaitClocks = 6000000000ll;  // about 3 s of waiting at most (FEA_WAIT_CLOCKS: another bound)
 constexpr int64_t kResidentSteps = 256;          // steps of one launch at most
 constexpr int kMaxBlocks = 160;                  // slots per value of the partials' buffers
 constexpr int kClusterBlocks = 16;               // blocks of a cluster launch (above 8: opt-in)
@@ -118,16 +119,24 @@ __device__ __forceinline__ bool try_get(const uint2* buf, int64_t i, T& v, uint3
     return ok;
 }
 
+// How long a wait may last, and where a block notes that one expired.
+struct Patience {
+    volatile int* dead;
+    long long most;
+    __device__ __forceinline__ bool over(long long since) const {
+        if (!*dead && clock64() - since <= most) return false;
+        *dead = 1;
+        return true;
+    }
+};
+
 template <typename T>
-__device__ __forceinline__ T get(const uint2* buf, int64_t i, uint32_t epoch, volatile int* dead) {
+__device__ __forceinline__ T get(const uint2* buf, int64_t i, uint32_t epoch, const Patience& wait) {
     T v;
     if (try_get(buf, i, v, epoch)) return v;
     const long long t0 = clock64();
     while (!try_get(buf, i, v, epoch))
-        if (*dead || clock64() - t0 > kWaitClocks) {
-            *dead = 1;
-            break;
-        }
+        if (wait.over(t0)) break;
     return v;
 }
 
@@ -136,7 +145,7 @@ __device__ __forceinline__ T get(const uint2* buf, int64_t i, uint32_t epoch, vo
 // Gray-Scott on a 251 x 251 grid (124 blocks) took 7,640 us against 6,320, and
 // heat on a 550 x 550 grid (four passes) 27,570 against 20,140.
 template <int n, typename T, typename Want, typename Try>
-__device__ __forceinline__ void get_all(T (&v)[n], Want want, Try attempt, volatile int* dead) {
+__device__ __forceinline__ void get_all(T (&v)[n], Want want, Try attempt, const Patience& wait) {
     bool here[n];
 #pragma unroll
     for (int i = 0; i < n; i++) here[i] = !want(i);
@@ -155,10 +164,7 @@ __device__ __forceinline__ void get_all(T (&v)[n], Want want, Try attempt, volat
         }
         if (all) return;
         if (t0 == 0) t0 = clock64();
-        if (*dead || clock64() - t0 > kWaitClocks) {
-            *dead = 1;
-            return;
-        }
+        if (wait.over(t0)) return;
     }
 }
 
@@ -173,7 +179,7 @@ __device__ __forceinline__ void put_remote(uint2* p, int rank, const uint2& v, u
     asm volatile("st.relaxed.cluster.shared::cluster.v2.u32 [%0], {%1, %2};" ::"r"(at + 8), "r"(v.y), "r"(epoch)
                  : "memory");
 }
-__device__ __forceinline__ uint2 get_shared(const uint2* p, uint32_t epoch, volatile int* dead) {
+__device__ __forceinline__ uint2 get_shared(const uint2* p, uint32_t epoch, const Patience& wait) {
     const uint32_t at = (uint32_t)__cvta_generic_to_shared(p);
     uint2 v;
     uint32_t e0, e1;
@@ -186,10 +192,7 @@ __device__ __forceinline__ uint2 get_shared(const uint2* p, uint32_t epoch, vola
                      : "memory");
         if (e0 == epoch && e1 == epoch) return v;
         if (t0 == 0) t0 = clock64();
-        if (*dead || clock64() - t0 > kWaitClocks) {
-            *dead = 1;
-            return v;
-        }
+        if (wait.over(t0)) return v;
     }
 }
 __device__ __forceinline__ void cluster_barrier() {
@@ -254,6 +257,8 @@ struct ResidentArgs {
     int T, tpb;              // tiles per block, tiles a block works on at a time
     int cluster;             // the blocks are one cluster
     int us;                  // staged operands per tile: kTileRows + the largest halo
+    long long left;          // steps of the call from this launch's first on
+    long long wait;          // clocks a wait may last
     const R* Ks;             // tile-ELL copies of K and Adv (M: StepArgs::Ms)
     const R* Advs;
     const int32_t* where;    // stiff groups: 4 * group + place of a row, -1 elsewhere
@@ -334,6 +339,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
             if (hcol[q] >= 0) hd[q] = ldfv(a.dinv_it + hcol[q]);
         }
     }
+    const Patience wait{&dead, ra.wait};
     auto ub_of = [&](int q) FEA_INLINE { return ub + (q * ra.tpb + grp) * us; };
     // outside the iterations: the thread's row and tile, addresses not kept
     auto row_of = [&](int q) FEA_INLINE { return (int64_t)opaque(rowq[q]); };
@@ -369,7 +375,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
                 if (l < nb) put_remote(&part[ph][w][blockIdx.x][0], l, bits, ep);
                 y = A();
                 if (l < nb) {
-                    bits = get_shared(&part[ph][w][l][0], ep, &dead);
+                    bits = get_shared(&part[ph][w][l][0], ep, wait);
                     memcpy(&mine, &bits, 8);
                     y = A::unpack(mine);
                 }
@@ -382,7 +388,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
                     Pk v[B];
                     get_all<B, Pk>(
                         v, [&](int u) FEA_INLINE { return l + 32 * u < nb; },
-                        [&](int u, Pk& x) FEA_INLINE { return try_get<Pk>(slots, l + 32 * u, x, ep); }, &dead);
+                        [&](int u, Pk& x) FEA_INLINE { return try_get<Pk>(slots, l + 32 * u, x, ep); }, wait);
                     y = A();
 #pragma unroll
                     for (int u = 0; u < B; u++)
@@ -396,9 +402,9 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
             if (l == 0 && (ra.cluster || blockIdx.x == 0)) reinterpret_cast<Pk*>(tot)[w] = y.pack();
         }
         if (!ra.cluster && blockIdx.x != 0 && threadIdx.x < N)
-            reinterpret_cast<Pk*>(tot)[threadIdx.x] = get<Pk>(sums + (blockIdx.x & 7) * 64, threadIdx.x, ep, &dead);
+            reinterpret_cast<Pk*>(tot)[threadIdx.x] = get<Pk>(sums + (blockIdx.x & 7) * 64, threadIdx.x, ep, wait);
         ph ^= 1;
-        return __syncthreads_or(*(volatile int*)&dead) == 0;  // the same answer in every thread
+        return __syncthreads_or(*wait.dead) == 0;  // the same answer in every thread
     };
     auto x_epoch = [&]() FEA_INLINE { return ++epoch != 0 ? epoch : ++epoch; };  // (0 has a meaning, below)
     auto total = [&](int k) FEA_INLINE { return Acc<R>::unpack(reinterpret_cast<typename Acc<R>::Packed*>(tot)[k]); };
@@ -459,12 +465,12 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
         const bool extrap = prev_ok && run->guess == 1;
         const int xb = step & 1;  // x buffer of this step's result; the other holds x_n
         auto state = [&](int64_t i, bool halo) FEA_INLINE {  // x_n of row i
-            return halo && xep[xb ^ 1] ? get<V>(ra.xl[xb ^ 1], i, xep[xb ^ 1], &dead) : ldv(a.x + i, true);
+            return halo && xep[xb ^ 1] ? get<V>(ra.xl[xb ^ 1], i, xep[xb ^ 1], wait) : ldv(a.x + i, true);
         };
         auto guess = [&](const V& xn, int64_t i, bool halo) FEA_INLINE {  // the solve's start there
             V g = xn;
             if (extrap) {
-                const V xp = halo && xep[xb] ? get<V>(ra.xl[xb], i, xep[xb], &dead) : ldv(a.xprev + i, true);
+                const V xp = halo && xep[xb] ? get<V>(ra.xl[xb], i, xep[xb], wait) : ldv(a.xprev + i, true);
 #pragma unroll
                 for (int f = 0; f < NF; f++) g.v[f] = fmar((R)2, xn.v[f], -xp.v[f]);
             }
@@ -522,7 +528,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
         if (wave) {
             const R c2 = (R)prm.c2;
             stage([&](int q, int64_t) FEA_INLINE { return cx[q]; },
-                  [&](int64_t i) FEA_INLINE { return get<V>(ra.yl, i, wep, &dead); });
+                  [&](int64_t i) FEA_INLINE { return get<V>(ra.yl, i, wep, wait); });
             add_term(ra.Ks, [&](R m) FEA_INLINE { return -c2 * m; });
         }
         if constexpr (NF == 2) {
@@ -648,7 +654,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
                         for (int i = 0; i < 4; i++) {
                             const int m = __ldg(a.grp_mem + (wr & ~3) + i);
                             if (m < 0) continue;
-                            const V rm = get<V>(ra.rl[0], m, rep, &dead);
+                            const V rm = get<V>(ra.rl[0], m, rep, wait);
 #pragma unroll
                             for (int f = 0; f < NF; f++)
                                 s[f] += a.grp_Q[16 * ((int64_t)(wr >> 2) * NF + f) + 4 * i + (wr & 3)] * (double)rm.v[f];
@@ -699,7 +705,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
                     for (int f = 0; f < NF; f++) z.v[f] = cd[q].v[f] * cr[q].v[f];
                     if (tile_of(q) >= 0) u[t] = z;
                     if (hcol[q] >= 0) {
-                        hr[q] = get<V>(rsrc, hcol[q], hep, &dead);
+                        hr[q] = get<V>(rsrc, hcol[q], hep, wait);
 #pragma unroll
                         for (int f = 0; f < NF; f++) z.v[f] = hd[q].v[f] * hr[q].v[f];
                         u[kTileRows + j] = z;
@@ -750,7 +756,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
                     // the halos' w, wanted after the rows' updates
                     get_all<kP, V>(
                         hw, [&](int q) FEA_INLINE { return hcol[q] >= 0; },
-                        [&](int q, V& x) FEA_INLINE { return try_get<V>(ra.wl[k & 1], hcol[q], x, wep2); }, &dead);
+                        [&](int q, V& x) FEA_INLINE { return try_get<V>(ra.wl[k & 1], hcol[q], x, wep2); }, wait);
                     PhaseCtl<R, NF> c;
                     c.need_old = k > 0;
 #pragma unroll
@@ -899,7 +905,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
                         for (int i = 0; i < 4; i++) {
                             const int m = __ldg(a.grp_mem + (wr & ~3) + i);
                             if (m < 0) continue;
-                            const V y = get<V>(ra.rl[1], m, yep, &dead);
+                            const V y = get<V>(ra.rl[1], m, yep, wait);
 #pragma unroll
                             for (int f = 0; f < NF; f++)
                                 s[f] += a.grp_Q[16 * ((int64_t)(wr >> 2) * NF + f) + 4 * (wr & 3) + i] * (double)y.v[f];
@@ -912,7 +918,10 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
                         for (int f = 0; f < NF; f++)
                             if (was[f]) st.thr[f] = solve_threshold<R>(run->tol, st.bb[f]);
                 }
-                __syncthreads();
+                if (__syncthreads_or(*wait.dead)) {  // (the members' values came after the last reduction)
+                    failed = true;
+                    break;
+                }
             }
             // x to global memory and to the halos; zero right-hand sides give x = 0
             xep[xb] = x_epoch();
@@ -930,7 +939,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
             if (round > 0 || !mode || st.iter >= st.max_iter) break;
             rep = ++epoch;
             stage([&](int q, int64_t) FEA_INLINE { return cx[q]; },
-                  [&](int64_t i) FEA_INLINE { return get<V>(ra.xl[xb], i, xep[xb], &dead); });
+                  [&](int64_t i) FEA_INLINE { return get<V>(ra.xl[xb], i, xep[xb], wait); });
             auto residual = [&](auto tag) FEA_INLINE -> bool {
                 using A = decltype(tag);
                 A dots[2 * NF];
@@ -1013,9 +1022,12 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
             }
     }
     if (ra.cluster) cluster_barrier();  // no block leaves while another may write into it
-    if (dead) {
-        if (threadIdx.x == 0) atomicOr(&run->flags, FEA_STATUS_BREAKDOWN);
-        halt = 1;
+    // a wait expired here: whichever block it was, the call's later launches do
+    // nothing and its step count leaves out the steps this block did not finish
+    if (dead && threadIdx.x == 0) {
+        atomicOr(&run->flags, FEA_STATUS_BREAKDOWN);
+        atomicExch(&run->halt, 1);
+        atomicMax(&run->lost, ra.left - done);
     }
     // has_numerical_instability of the final state (k_final_check)
     unsigned int flags = 0;
@@ -1035,7 +1047,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
     raise_flags(run, flags);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         if (sflags) atomicOr(&run->flags, sflags);
-        if (halt) run->halt = 1;
+        if (halt) atomicExch(&run->halt, 1);
         run->epoch = epoch + (dead ? 1u << 20 : 0u);  // past anything another block may have sent
         run->steps_done = (ra.first ? 0 : run->steps_done) + done;
         run->steps_left = 0;
@@ -1171,8 +1183,12 @@ void run_resident(const StepArgs<R, NF>& a, const ResidentPlan& p, const R* Ks, 
     ra.cluster = p.cluster;
     cudaLaunchAttribute attr;
     const cudaLaunchConfig_t cfg = launch_config(p, attr, st);
-    FEA_CUDA_TRY(cudaMemsetAsync(&a.run->flags, 0, 2 * sizeof(unsigned int), st));  // and the halt word
+    ra.wait = kWaitClocks;
+    if (const char* most = getenv("FEA_WAIT_CLOCKS"))
+        if (const long long n = strtoll(most, nullptr, 10); n > 0) ra.wait = n;
+    FEA_CUDA_TRY(cudaMemsetAsync(&a.run->flags, 0, kRunFlagBytes, st));
     for (int64_t s0 = 0; s0 < nsteps; s0 += kResidentSteps) {
+        ra.left = nsteps - s0;
         ra.first = s0 == 0;
         ra.steps = (int)std::min<int64_t>(kResidentSteps, nsteps - s0);
         FEA_CUDA_TRY(cudaLaunchKernelEx(&cfg, fn, a, ra));

@@ -239,6 +239,7 @@ struct fea_solver {
     int* grp_in = nullptr;
     bool diagonal_only = false;     // solves without the stiff groups, on the step graph (DiagonalOnly)
     void *Ks_ell = nullptr, *Advs_ell = nullptr;               // tile-ELL copies of K and Adv (resident launches)
+    int64_t run_steps = 0;          // steps asked of the last resident run
     bool resident = true;           // the step loop may run as one resident launch (no CG variant chosen)
     struct {
         int known = 0;              // 0: not asked, 1: fits, -1: does not
@@ -831,6 +832,7 @@ bool try_resident(fea_solver* s, const StepArgs<R, NF>& a, int kind, int64_t nst
         ex = s->mat_mem.alloc<unsigned char>((int64_t)n);
         FEA_CUDA_TRY(cudaMemsetAsync(ex, 0, n, s->stream));
     }
+    s->run_steps = nsteps;
     run_resident<R, NF>(a, *p, (const R*)s->Ks_ell, (const R*)s->Advs_ell, s->grp.where, ex, kind, nsteps, s->stream);
     return true;
 }
@@ -850,7 +852,7 @@ void run_graph(fea_solver* s, StepGraph& g, int kind, bool init_op, int64_t nste
     }
     long long ctl[2] = {nsteps, 0};  // steps_left, steps_done
     FEA_CUDA_TRY(cudaMemcpyAsync(s->d_run, ctl, sizeof(ctl), cudaMemcpyHostToDevice, s->stream));
-    FEA_CUDA_TRY(cudaMemsetAsync(&s->d_run->flags, 0, sizeof(unsigned int), s->stream));
+    FEA_CUDA_TRY(cudaMemsetAsync(&s->d_run->flags, 0, kRunFlagBytes, s->stream));
     if (stream_mode) {
         StepArgs<R, NF> a = make_args<R, NF>(s, init_op);
         set_x<R, NF>(s, a, kind);
@@ -1012,7 +1014,7 @@ void run_given(fea_solver* s, const StepArgs<R, NF>& a) {
     if (try_resident<R, NF>(s, a, EQ_GIVEN, 1)) return;
     long long ctl[2] = {1, 0};  // steps_left, steps_done
     FEA_CUDA_TRY(cudaMemcpyAsync(s->d_run, ctl, sizeof(ctl), cudaMemcpyHostToDevice, s->stream));
-    FEA_CUDA_TRY(cudaMemsetAsync(&s->d_run->flags, 0, sizeof(unsigned int), s->stream));
+    FEA_CUDA_TRY(cudaMemsetAsync(&s->d_run->flags, 0, kRunFlagBytes, s->stream));
     if (s->stream_mode) {
         run_steps_stream<R, NF>(a, EQ_GIVEN, s->lanes, s->d_flags, s->stream);
         return;
@@ -1948,7 +1950,7 @@ int fea_get_status(fea_solver* s, fea_status* out) {
     out->last_iterations[1] = r.last_iters[1];
     out->last_rel_residual[0] = r.last_rel[0];
     out->last_rel_residual[1] = r.last_rel[1];
-    out->steps_done = r.steps_done;
+    out->steps_done = r.lost > 0 ? std::min<int64_t>(r.steps_done, s->run_steps - r.lost) : r.steps_done;
     out->total_iterations = r.total_iters;
     out->cg_launches = r.cg_launches;
     API_END
