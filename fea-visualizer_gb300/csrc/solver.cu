@@ -191,6 +191,19 @@ struct Scratch {
     }
 };
 
+// The states of an adjoint sweep: one field per checkpoint and per step of a
+// segment, a count the caller chooses.  They go back to the device after a
+// sweep that needed more than kStatesKept; below that the handle keeps them
+// (freeing and allocating them cost 0.1 ms a buffer and a wait for the device).
+constexpr int64_t kStatesKept = (int64_t)64 << 20;
+struct SweepStates {
+    Scratch& mem;
+    explicit SweepStates(Scratch& m) : mem(m) { mem.rewind(); }
+    ~SweepStates() {
+        if (mem.bytes() > kStatesKept) mem.release();
+    }
+};
+
 }  // namespace fea
 
 using namespace fea;
@@ -264,7 +277,7 @@ struct fea_solver {
     struct {
         const void *x = nullptr, *rhs = nullptr, *op = nullptr;
     } given_for[2];
-    Scratch scratch[3];  // adjoint sweeps, their entry points, smooth normals
+    Scratch scratch[4];  // adjoint sweeps, their entry points, smooth normals, the sweeps' states
     int lanes = 8;  // CG kernel variant: 0/1 tile-ELL (8/4 entries prefetched), 2/3 streamed (stages), 4/8/16 CSR window
     bool op_dirty = true;
     int op_kind = -1;
@@ -1045,10 +1058,11 @@ double adjoint_core(fea_solver* s, const R* u0, const R* t, int64_t nsteps, int6
     ckpt = std::min(ckpt, nsteps);
     const int64_t nck = ceil_div(nsteps, ckpt);
     ensure_layout<R>(s, false);
+    const SweepStates states(s->scratch[3]);
     Scratch& tmp = s->scratch[0];
     tmp.rewind();
-    R* ck = tmp.alloc<R>(nck * N);
-    R* seg = tmp.alloc<R>((ckpt + 1) * N);
+    R* ck = states.mem.alloc<R>(nck * N);
+    R* seg = states.mem.alloc<R>((ckpt + 1) * N);
     R* mu = tmp.alloc<R>(pad_tiles(N));  // x of the solves: whole tiles
     R* uN = tmp.alloc<R>(N);
     R* lam_f = lam ? lam : tmp.alloc<R>(N);
@@ -1114,10 +1128,11 @@ double adjoint_gs_core(fea_solver* s, const FV<R, 2>* x0, const FV<R, 2>* t, int
     ckpt = std::min(ckpt, nsteps);
     const int64_t nck = ceil_div(nsteps, ckpt);
     ensure_layout<R>(s, true);  // the forward steps update the operator to the current parameters
+    const SweepStates states(s->scratch[3]);
     Scratch& tmp = s->scratch[0];
     tmp.rewind();
-    FV<R, 2>* ck = tmp.alloc<FV<R, 2>>(nck * N);
-    FV<R, 2>* seg = tmp.alloc<FV<R, 2>>((ckpt + 1) * N);
+    FV<R, 2>* ck = states.mem.alloc<FV<R, 2>>(nck * N);
+    FV<R, 2>* seg = states.mem.alloc<FV<R, 2>>((ckpt + 1) * N);
     FV<R, 2>* mu = tmp.alloc<FV<R, 2>>(pad_tiles(N));  // x of the solves: whole tiles
     FV<R, 2>* xN = tmp.alloc<FV<R, 2>>(N);
     double* J = tmp.alloc<double>(1);
