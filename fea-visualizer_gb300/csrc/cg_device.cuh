@@ -6,6 +6,7 @@
 #include <tuple>
 
 #include "fea_internal.cuh"
+#include "shared_limit.h"
 
 namespace fea {
 namespace {
@@ -896,16 +897,23 @@ cudaGraphNode_t add_while(cudaGraph_t g, cudaGraphNode_t dep, cudaGraphCondition
 }
 
 // Opts `kernel` in to `smem` bytes of dynamic shared memory when that is above
-// its current limit (48 KB less its static shared memory at first).  The limit is a property of the function, shared by
-// every handle, so it only ever grows: a graph instantiated for a larger
-// handle stays launchable after a smaller one is set up.
+// its current limit (48 KB less its static shared memory at first).  The limit
+// is a property of the function, shared by every handle and thread, so it only
+// ever grows: a launch or graph set up for a larger handle stays valid after a
+// smaller one is set up.
 template <typename K>
 void ensure_dyn_smem(K kernel, size_t smem) {
     if (smem == 0) return;
-    cudaFuncAttributes fa{};
-    FEA_CUDA_TRY(cudaFuncGetAttributes(&fa, kernel));
-    if ((size_t)fa.maxDynamicSharedSizeBytes < smem)
-        FEA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    raise_shared_limit(
+        smem,
+        [&] {
+            cudaFuncAttributes fa{};
+            FEA_CUDA_TRY(cudaFuncGetAttributes(&fa, kernel));
+            return (size_t)fa.maxDynamicSharedSizeBytes;
+        },
+        [&](size_t n) {
+            FEA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)n));
+        });
 }
 
 // Grid of one wave: SMs x resident blocks of this kernel (from the occupancy
