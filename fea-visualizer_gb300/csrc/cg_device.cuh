@@ -272,32 +272,6 @@ __device__ __forceinline__ void merge_partials(Acc<R> (&y)[NV], const typename A
     }
 }
 
-// Totals of NV values over nb block partials p[k * stride + b]: warp k merges
-// value k (lane l takes b = l, l + 32, ... with 16 loads in flight, then a
-// shuffle tree), a fixed order; lane 0 of warp k leaves total k in sm[k].
-// Needs NV <= the block's warps; every thread calls it (no barrier inside).
-template <int NV, typename R>
-__device__ __forceinline__ void merge_partials_by_warp(const typename Acc<R>::Packed* p, int64_t stride, int nb,
-                                                       typename Acc<R>::Packed* sm) {
-    using P = typename Acc<R>::Packed;
-    constexpr int B = 16;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (w >= NV) return;
-    Acc<R> y;
-    for (int base = lane; base < nb; base += 32 * B) {
-        P v[B];
-#pragma unroll
-        for (int u = 0; u < B; u++)
-            if (base + 32 * u < nb) v[u] = __ldcg(&p[w * stride + base + 32 * u]);
-#pragma unroll
-        for (int u = 0; u < B; u++)
-            if (base + 32 * u < nb) y.merge(Acc<R>::unpack(v[u]));
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) y.shfl_add(o);
-    if (lane == 0) sm[w] = y.pack();
-}
-
 // Last-block-done reduction of block totals held in thread 0: every block
 // stores its NV totals, packed, to part[k * stride + blockIdx.x] (8-byte
 // slots); the block that finishes last merges all partials in a fixed order

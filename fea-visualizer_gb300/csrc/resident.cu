@@ -1066,10 +1066,13 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
 template <typename R, int NF>
 using ResidentFn = void (*)(StepArgs<R, NF>, ResidentArgs<R>);
 
-// The kernel for `passes` tiles per thread group, or null: as many passes as
-// the 128 registers hold (9 to 36 of them per pass by type and fields).  At 17 tiles
-// a block (the level-8 icosphere, one FP32 field) nine passes ran 50 Newmark
-// steps in 16.5 ms, the step graph in 10.0.
+// The kernel for `passes` tiles per thread group, or null: up to where the step
+// graph is faster.  A pass keeps 9 to 36 registers by type and fields, and every
+// instance uses all 128 of a thread and spills the rest
+// (bytes of spill stores for one pass and for the most:
+// FP32 one field 204 and 396, two fields 244 and 1004, FP64 one field 0 and 432, two
+// fields 92 and 408).  At 17 tiles a block (the level-8 icosphere, one FP32
+// field) nine passes ran 50 Newmark steps in 16.5 ms, the step graph in 10.0.
 template <typename R, int NF>
 ResidentFn<R, NF> resident_kernel(int passes) {
     if (passes <= 1) return k_resident<R, NF, 1>;

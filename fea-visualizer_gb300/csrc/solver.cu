@@ -552,11 +552,15 @@ void build_context(fea_solver* s) {
     FEA_CUDA_TRY(cudaStreamSynchronize(st));
 }
 
-// The FP32 wave on larger meshes: its velocity sums accelerations -c^2 M^-1 K u
-// whose FP32 rounding grows with the mesh (7e-5 of the velocity against FP64
-// on the 500 x 500 grid, whatever the solver), and a different order of the
-// sums moves it by a third of that.  Such handles keep the diagonal iteration
-// on the step graph, bit for bit.
+// The FP32 wave on larger meshes keeps the diagonal iteration on the step graph,
+// bit for bit: its velocity sums accelerations -c^2 M^-1 K u whose FP32 rounding
+// grows with the mesh, and another order of the sums moves it by a large part of
+// that error.  Ten Newmark steps, four starts, velocity against 64 bits with this
+// rule and without it (groups; the resident launch where it fits), and how far the two are apart:
+// grid 200 x 200 3.1 to 6.1e-5 either way, apart 0.9 to 1.7e-5; 500 x 500 7.0e-5 to
+// 1.7e-4 against 6.7e-5 to 1.6e-4, apart 4.5 to 8.3e-5; 900 x 900 9.1e-5 to 2.8e-4
+// against 8.7e-5 to 2.3e-4, apart 6.3e-5 to 2.0e-4.  So the rule keeps bits, not
+// accuracy; without it those runs take 1.3 ms for 2.6, 2.3 for 10 and 7.5 for 33.
 bool rounding_bound_wave(const fea_solver* s) {
     return s->precision == FEA_FP32 && s->prm.equation == FEA_WAVE && s->N > 16384;
 }
@@ -800,10 +804,14 @@ struct GuessOff {
     }
 };
 
-// Solves without the stiff groups and on the step graph while it lives: the
-// FP32 Gray-Scott adjoint returns FP64 parameter gradients, sums over FP32
-// fields whose last digits follow the iteration's rounding, and keeps the
-// iteration it was validated with.
+// Solves without the stiff groups and on the step graph while it lives: the FP32
+// Gray-Scott adjoint keeps the bits of the iteration it was validated with, its
+// FP64 parameter gradients included.  Against 64 bits, four starts, with this and
+// without it: loss on the 400 x 400 grid 0.3 to 4.1e-7 against 4.3 to 6.0e-7, on 512
+// x 512 3.8e-7 to 1.2e-6 against 2.9 to 9.4e-7; dJ/du0 4.6 to 5.8e-6 against 4.0 to
+// 4.4e-6, and 5.9 to 9.1e-6 against 7.7 to 8.3e-6; the four rates 0.9 to 8.7e-7 against
+// 2.3 to 7.4e-7, and 3.4e-7 to 2.3e-6 against 2.2e-7 to 2.6e-6.  Neither is the more
+// accurate throughout; without it a 512 x 512 sweep takes 22 ms for 53.
 struct DiagonalOnly {
     fea_solver* s;
     DiagonalOnly(fea_solver* h, bool on) : s(h) { s->diagonal_only = on; }

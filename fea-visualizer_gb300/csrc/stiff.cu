@@ -24,9 +24,9 @@
 // one widens its neighbours' rows.  A uniformly stretched grid stays below
 // 0.6, so anisotropic meshes are left alone.  Groups of more than four
 // changed no iteration count.  On the GPU, 10 steps of the 1024 x 1024 Gray-
-// Scott workload (about 800 unknowns of 1,048,576 in groups) take 19.6 ms
-// against 46.2 ms without groups, the FP64 advection-diffusion adjoint of the 512
-// x 512 grid 76 against 148 ms.
+// Scott workload (about 800 unknowns of 1,048,576 in groups) take 19.9 ms
+// against 46.4 ms without groups, the FP64 advection-diffusion adjoint of the 512
+// x 512 grid 65.5 against 145 ms (both with this library's other changes of then).
 #include <algorithm>
 #include <array>
 #include <unordered_map>
@@ -37,10 +37,12 @@ namespace fea {
 namespace {
 
 constexpr double kStiffBound = 0.75;
-// Meshes with fewer groups keep the diagonal iteration.  20 Gray-Scott steps
-// of the 251 x 251 grid (19 groups): 9.6 ms without groups, 10.6 ms with them
-// (62 against 65 iterations a step at the loop's tighter stop, and four small
-// launches); 8 steps of the 500 x 500 grid (about 95): 14.1 against 8.0 ms.
+// Meshes with fewer groups keep the diagonal iteration, whose loop stops at the
+// tolerance itself.  Gray-Scott on jittered grids, resident launch, groups against
+// none (iterations a step): 251 x 251, 22 groups, 20 steps 6.73 against 6.09 ms (65
+// / 62); 330 x 330, 21 groups, 10 steps 4.64 against 5.45 (74 / 92); 500 x 500, 89
+// groups, 8 steps 6.81 against 13.39 (75 / 177).  On the step graph 10.06 against
+// 9.61, 6.79 against 8.01, 7.22 against 15.22.  Some 20 groups may go either way.
 constexpr int kFewestGroups = 32;
 // Smaller meshes are not searched: their solves are bound by launches, and the
 // search would add a tenth of a millisecond to opening them.

@@ -48,7 +48,8 @@ extern "C" {
 #define FEA_STATUS_BLOWUP 1u       /* some u_i or v_i > 1e4 (CPUSolver.cpp:41-48) */
 #define FEA_STATUS_NONFINITE 2u    /* NaN or Inf in a field */
 #define FEA_STATUS_NOT_CONVERGED 4u /* a CG solve hit max_iter before tol */
-#define FEA_STATUS_BREAKDOWN 8u    /* CG breakdown: p.Ap <= 0 or non-finite */
+#define FEA_STATUS_BREAKDOWN 8u    /* CG breakdown: p.Ap <= 0 or non-finite; or a wait
+                                      between a kernel's blocks expired */
 
 /* ---- enums mirroring the reference --------------------------------------- */
 /* Equation, include/FEM/FEMContext.hpp:9-14 (same order and values) */
@@ -134,7 +135,8 @@ typedef struct {
     int precision;               /* FEA_FP32 / FEA_FP64 */
     int boundary_condition;
     int rows_per_warp_lanes;     /* CG kernel variant (fea_set_cg_variant, fea_autotune) */
-    int64_t device_bytes;        /* device memory held by the handle */
+    int64_t device_bytes;        /* device memory held by the handle, work arrays kept
+                                    between calls included */
 } fea_info;
 
 typedef struct {
