@@ -110,6 +110,12 @@ __global__ void k_compose_idx(const int32_t* __restrict__ idx, const int32_t* __
         idx_c[i] = idx[i] >= 0 ? pos[idx[i]] : -1;
 }
 
+// *found = 1 when an unknown has no mass: no triangle, or none with an area.
+__global__ void k_bare_rows(int64_t N, const int32_t* __restrict__ diag, const double* __restrict__ M, int* found) {
+    for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < N; u += (int64_t)gridDim.x * blockDim.x)
+        if (diag[u] < 0 || !(M[diag[u]] > 0)) *found = 1;
+}
+
 template <typename R>
 __global__ void k_float_to(const float* __restrict__ in, int64_t n, R* out) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -253,6 +259,7 @@ struct fea_solver {
     bool diagonal_only = false;     // solves without the stiff groups, on the step graph (DiagonalOnly)
     void *Ks_ell = nullptr, *Advs_ell = nullptr;               // tile-ELL copies of K and Adv (resident launches)
     int64_t run_steps = 0;          // steps asked of the last resident run
+    int bare = -1;                  // unknowns without mass (bare_rows): -1 not asked
     bool resident = true;           // the step loop may run as one resident launch (no CG variant chosen)
     struct {
         int known = 0;              // 0: not asked, 1: fits, -1: does not
@@ -441,6 +448,7 @@ void build_context(fea_solver* s) {
     s->S1 = s->S0 = s->S2 = nullptr;
     s->S1d = s->S0d = s->S2d = nullptr;
     s->Ms_ell = nullptr;
+    s->bare = -1;
     s->grp = StiffGroups{};
     s->ell_st = TileEll{};
     s->Ks_ell = s->Advs_ell = nullptr;
@@ -565,6 +573,32 @@ bool rounding_bound_wave(const fea_solver* s) {
     return s->precision == FEA_FP32 && s->prm.equation == FEA_WAVE && s->N > 16384;
 }
 
+// Whether some unknown of the mesh has no mass, as a vertex that no triangle
+// names (asked once per assembly, by the equation it matters to).
+bool bare_rows(fea_solver* s) {
+    if (s->bare < 0) {
+        DeviceArena tmp;
+        int* found = tmp.alloc<int>(1);
+        FEA_CUDA_TRY(cudaMemsetAsync(found, 0, sizeof(int), s->stream));
+        k_bare_rows<<<launch_grid(s->N), kBlock, 0, s->stream>>>(s->N, s->P.diag, s->M64, found);
+        FEA_CHECK_LAUNCH();
+        int h = 0;
+        FEA_CUDA_TRY(cudaMemcpyAsync(&h, found, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+        FEA_CUDA_TRY(cudaStreamSynchronize(s->stream));
+        s->bare = h;
+    }
+    return s->bare > 0;
+}
+
+// The nodal reaction (the reference's) on a mesh with such unknowns: their
+// equations read 0 = reaction, the system has no solution, and the step graph's
+// diagonal iteration reports it (the value runs away past 1e4, as it does
+// under the reference's CG).  Started from the diagonal-free product, as the
+// resident launch and the groups do, CG would take the row's diagonal for 1 and
+// converge on a value that solves nothing.  Under every other equation such a row's
+// right-hand side is 0.
+bool nodal_on_bare_rows(fea_solver* s) { return step_kind(s->prm) == EQ_GS_REF && bare_rows(s); }
+
 // Whether variant l iterates in the basis of the handle's stiff groups.
 bool stiff_variant(const fea_solver* s, int l) {
     return s->grp.n > 0 && is_ring_variant(l) && ring_fits(s, s->ell_st, ring_stages(l));
@@ -573,10 +607,10 @@ bool stiff_variant(const fea_solver* s, int l) {
 // Whether the current equation's solves run in the stiff groups' basis.
 // Implicit advection-diffusion does not: its operator is not symmetric, CG
 // may break down on it, and it keeps the iteration it had.
-bool stiff_solves(const fea_solver* s) {
+bool stiff_solves(fea_solver* s) {
     if (rounding_bound_wave(s)) return false;
     const bool symmetric = s->prm.equation != FEA_ADVECTION_DIFFUSION || s->prm.advection_scheme == 1;
-    return stiff_variant(s, s->lanes) && !s->diagonal_only && symmetric;
+    return stiff_variant(s, s->lanes) && !s->diagonal_only && symmetric && !nodal_on_bare_rows(s);
 }
 
 // r, w and s of the Chronopoulos-Gear iteration, two buffers each, carved
@@ -837,7 +871,9 @@ void ensure_layout(fea_solver* s, bool interleaved) {
 // The resident launch's shape for these arguments, or null: the step graph.
 template <typename R, int NF>
 const ResidentPlan* resident_plan(fea_solver* s, const StepArgs<R, NF>& a) {
-    if (!s->resident || s->stream_mode || s->diagonal_only || !s->Ks_ell || rounding_bound_wave(s)) return nullptr;
+    if (!s->resident || s->stream_mode || s->diagonal_only || !s->Ks_ell || rounding_bound_wave(s) ||
+        nodal_on_bare_rows(s))
+        return nullptr;
     auto& r = s->res[NF - 1][a.ngrp ? 1 : 0];
     if (r.known == 0) r.known = plan_resident<R, NF>(a, r.plan) ? 1 : -1;
     return r.known > 0 ? &r.plan : nullptr;
