@@ -188,10 +188,11 @@ struct CgState {
 struct RunState {
     long long steps_left, steps_done, total_iters;
     long long cg_launches;  // iteration kernels run (timing probes excluded)
-    // kRunFlagBytes from here on are cleared as a run starts
+    // cleared as a run starts; `expired` as a call's first one does
     unsigned int flags;
     int halt;             // resident launches: a launch of this call stopped early
     long long lost;       // resident launches: steps of the call an expired wait left undone in some block
+    int expired;          // resident launches: a wait expired in a run of this call
     unsigned int epoch;   // resident launches: the last exchange's number
     int last_iters[2];
     double last_rel[2];
@@ -202,7 +203,8 @@ struct RunState {
     int prev_valid;  // x_(n-1) of the extrapolation is the previous step's state
 };
 
-constexpr size_t kRunFlagBytes = offsetof(RunState, epoch) - offsetof(RunState, flags);
+constexpr size_t kCallFlagBytes = offsetof(RunState, epoch) - offsetof(RunState, flags);
+constexpr size_t kRunFlagBytes = offsetof(RunState, expired) - offsetof(RunState, flags);
 
 // Everything a step-loop kernel needs, passed by value.
 template <typename R, int NF>
@@ -324,7 +326,7 @@ bool plan_resident(const StepArgs<R, NF>& a, ResidentPlan& p);
 // Device memory through which a launch's blocks exchange (zeroed once).
 template <typename R, int NF>
 size_t resident_exchange_bytes(int64_t N);
-// nsteps steps of `kind` on the stream (Ks, Advs: tile-ELL copies of K and
+// nsteps steps of `kind` on the stream, the run's flags cleared before (Ks, Advs: tile-ELL copies of K and
 // Adv; where: the stiff groups' places by row, or null).
 template <typename R, int NF>
 void run_resident(const StepArgs<R, NF>& a, const ResidentPlan& p, const R* Ks, const R* Advs, const int32_t* where,

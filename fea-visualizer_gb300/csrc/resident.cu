@@ -1027,6 +1027,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(StepArgs<R, NF> a, 
     if (dead && threadIdx.x == 0) {
         atomicOr(&run->flags, FEA_STATUS_BREAKDOWN);
         atomicExch(&run->halt, 1);
+        atomicExch(&run->expired, 1);
         atomicMax(&run->lost, ra.left - done);
     }
     // has_numerical_instability of the final state (k_final_check)
@@ -1189,7 +1190,6 @@ void run_resident(const StepArgs<R, NF>& a, const ResidentPlan& p, const R* Ks, 
     ra.wait = kWaitClocks;
     if (const char* most = getenv("FEA_WAIT_CLOCKS"))
         if (const long long n = strtoll(most, nullptr, 10); n > 0) ra.wait = n;
-    FEA_CUDA_TRY(cudaMemsetAsync(&a.run->flags, 0, kRunFlagBytes, st));
     for (int64_t s0 = 0; s0 < nsteps; s0 += kResidentSteps) {
         ra.left = nsteps - s0;
         ra.first = s0 == 0;

@@ -259,6 +259,7 @@ struct fea_solver {
     bool diagonal_only = false;     // solves without the stiff groups, on the step graph (DiagonalOnly)
     void *Ks_ell = nullptr, *Advs_ell = nullptr;               // tile-ELL copies of K and Adv (resident launches)
     int64_t run_steps = 0;          // steps asked of the last resident run
+    bool many_runs = false, later_run = false;  // a call of several runs, past its first (CallRuns)
     int bare = -1;                  // unknowns without mass (bare_rows): -1 not asked
     bool resident = true;           // the step loop may run as one resident launch (no CG variant chosen)
     struct {
@@ -868,6 +869,38 @@ void ensure_layout(fea_solver* s, bool interleaved) {
     F.interleaved = interleaved;
 }
 
+// The flags of the last run go as another starts.  A call of several runs
+// (Newmark's starting acceleration and its steps, an adjoint's solves) keeps
+// word of an expired wait through all of them (CallRuns).
+void clear_run_flags(fea_solver* s) {
+    FEA_CUDA_TRY(cudaMemsetAsync(&s->d_run->flags, 0, s->later_run ? kRunFlagBytes : kCallFlagBytes, s->stream));
+    if (s->many_runs) s->later_run = true;
+}
+struct CallRuns {
+    fea_solver* s;
+    bool outer;  // (the adjoints' calls hold the steps' calls)
+    explicit CallRuns(fea_solver* h) : s(h), outer(!h->many_runs) {
+        if (outer) s->later_run = false;
+        s->many_runs = true;
+    }
+    ~CallRuns() {
+        if (outer) s->many_runs = s->later_run = false;
+    }
+};
+// The loss of a sweep, once no wait of its solves expired.
+double sweep_result(fea_solver* s, const double* J) {
+    double h = 0;
+    int expired = 0;
+    FEA_CUDA_TRY(cudaMemcpyAsync(&h, J, sizeof(double), cudaMemcpyDeviceToHost, s->stream));
+    FEA_CUDA_TRY(cudaMemcpyAsync(&expired, &s->d_run->expired, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+    FEA_CUDA_TRY(cudaStreamSynchronize(s->stream));
+    if (expired) {
+        set_error("a wait between the blocks of a solve expired");
+        throw Error{FEA_ERR_SOLVE};
+    }
+    return h;
+}
+
 // The resident launch's shape for these arguments, or null: the step graph.
 template <typename R, int NF>
 const ResidentPlan* resident_plan(fea_solver* s, const StepArgs<R, NF>& a) {
@@ -890,6 +923,7 @@ bool try_resident(fea_solver* s, const StepArgs<R, NF>& a, int kind, int64_t nst
         FEA_CUDA_TRY(cudaMemsetAsync(ex, 0, n, s->stream));
     }
     s->run_steps = nsteps;
+    clear_run_flags(s);
     run_resident<R, NF>(a, *p, (const R*)s->Ks_ell, (const R*)s->Advs_ell, s->grp.where, ex, kind, nsteps, s->stream);
     return true;
 }
@@ -909,7 +943,7 @@ void run_graph(fea_solver* s, StepGraph& g, int kind, bool init_op, int64_t nste
     }
     long long ctl[2] = {nsteps, 0};  // steps_left, steps_done
     FEA_CUDA_TRY(cudaMemcpyAsync(s->d_run, ctl, sizeof(ctl), cudaMemcpyHostToDevice, s->stream));
-    FEA_CUDA_TRY(cudaMemsetAsync(&s->d_run->flags, 0, kRunFlagBytes, s->stream));
+    clear_run_flags(s);
     if (stream_mode) {
         StepArgs<R, NF> a = make_args<R, NF>(s, init_op);
         set_x<R, NF>(s, a, kind);
@@ -932,6 +966,7 @@ void advance(fea_solver* s, int64_t nsteps) {
         s->op_kind = kind;
     }
     ensure_layout<R>(s, two_fields(kind));
+    const CallRuns runs(s);
     if (kind == EQ_WAVE_NEWMARK && !s->acc_valid) {
         // a0 from M a0 = -c^2 K u0
         FEA_CUDA_TRY(cudaMemsetAsync(s->F.a, 0, rsize(s) * (size_t)(s->N > 0 ? s->N : 1), s->stream));
@@ -1071,7 +1106,7 @@ void run_given(fea_solver* s, const StepArgs<R, NF>& a) {
     if (try_resident<R, NF>(s, a, EQ_GIVEN, 1)) return;
     long long ctl[2] = {1, 0};  // steps_left, steps_done
     FEA_CUDA_TRY(cudaMemcpyAsync(s->d_run, ctl, sizeof(ctl), cudaMemcpyHostToDevice, s->stream));
-    FEA_CUDA_TRY(cudaMemsetAsync(&s->d_run->flags, 0, kRunFlagBytes, s->stream));
+    clear_run_flags(s);
     if (s->stream_mode) {
         run_steps_stream<R, NF>(a, EQ_GIVEN, s->lanes, s->d_flags, s->stream);
         return;
@@ -1096,6 +1131,7 @@ double adjoint_core(fea_solver* s, const R* u0, const R* t, int64_t nsteps, int6
         throw Error{FEA_ERR_STATE};
     }
     cudaStream_t st = s->stream;
+    const CallRuns runs(s);
     const int64_t N = s->N;
     const size_t rb = sizeof(R) * (size_t)N;
     const auto d2d = cudaMemcpyDeviceToDevice;
@@ -1146,10 +1182,7 @@ double adjoint_core(fea_solver* s, const R* u0, const R* t, int64_t nsteps, int6
         }
     }
     FEA_CUDA_TRY(cudaMemcpyAsync(u, uN, rb, d2d, st));
-    double h = 0;
-    FEA_CUDA_TRY(cudaMemcpyAsync(&h, J, sizeof(double), cudaMemcpyDeviceToHost, st));
-    FEA_CUDA_TRY(cudaStreamSynchronize(st));
-    return h;
+    return sweep_result(s, J);
 }
 
 // ---- adjoint of the mass-weighted Gray-Scott step (kernels in adjoint.cu) ---------
@@ -1166,6 +1199,7 @@ double adjoint_gs_core(fea_solver* s, const FV<R, 2>* x0, const FV<R, 2>* t, int
     const GuessOff guess_off(s);  // recomputed forward states must equal the forward sweep's
     const DiagonalOnly diagonal(s, sizeof(R) == 4);
     cudaStream_t st = s->stream;
+    const CallRuns runs(s);
     const int64_t N = s->N;
     const size_t xb = sizeof(FV<R, 2>) * (size_t)N;
     const auto d2d = cudaMemcpyDeviceToDevice;
@@ -1218,10 +1252,7 @@ double adjoint_gs_core(fea_solver* s, const FV<R, 2>* x0, const FV<R, 2>* t, int
         }
     }
     FEA_CUDA_TRY(cudaMemcpyAsync(x, xN, xb, d2d, st));
-    double h = 0;
-    FEA_CUDA_TRY(cudaMemcpyAsync(&h, J, sizeof(double), cudaMemcpyDeviceToHost, st));
-    FEA_CUDA_TRY(cudaStreamSynchronize(st));
-    return h;
+    return sweep_result(s, J);
 }
 
 // Node-indexed float arrays (NULL targets drop their loss terms).
@@ -1898,7 +1929,7 @@ int fea_clear_values(fea_solver* s) {
     const size_t n = rsize(s) * (size_t)(s->N > 0 ? s->N : 1);
     for (void* p : {F.u, F.v, F.a}) FEA_CUDA_TRY(cudaMemsetAsync(p, 0, n, s->stream));
     FEA_CUDA_TRY(cudaMemsetAsync(F.uv, 0, 2 * n, s->stream));
-    FEA_CUDA_TRY(cudaMemsetAsync(&s->d_run->flags, 0, sizeof(unsigned int), s->stream));
+    FEA_CUDA_TRY(cudaMemsetAsync(&s->d_run->flags, 0, kCallFlagBytes, s->stream));
     s->acc_valid = false;
     invalidate_guess(s);
     FEA_CUDA_TRY(cudaStreamSynchronize(s->stream));
@@ -2004,7 +2035,7 @@ int fea_get_status(fea_solver* s, fea_status* out) {
     FEA_CUDA_TRY(cudaMemcpyAsync(s->h_run, s->d_run, sizeof(RunState), cudaMemcpyDeviceToHost, s->stream));
     FEA_CUDA_TRY(cudaStreamSynchronize(s->stream));
     const RunState& r = *s->h_run;
-    out->flags = r.flags;
+    out->flags = r.flags | (r.expired ? FEA_STATUS_BREAKDOWN : 0u);
     out->last_iterations[0] = r.last_iters[0];
     out->last_iterations[1] = r.last_iters[1];
     out->last_rel_residual[0] = r.last_rel[0];

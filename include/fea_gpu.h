@@ -42,7 +42,8 @@ extern "C" {
 #define FEA_ERR_STATE (-6)       /* call order violated (e.g. step before assemble) */
 #define FEA_ERR_UNSUPPORTED (-7)
 #define FEA_ERR_TOO_LARGE (-8)
-#define FEA_ERR_SOLVE (-9)       /* a solve broke down or met NaN/Inf (fea_pcg_solve_csr_noalloc) */
+#define FEA_ERR_SOLVE (-9)       /* a solve broke down or met NaN/Inf (fea_pcg_solve_csr_noalloc);
+                                    a wait between a kernel's blocks expired (adjoints) */
 
 /* ---- step status flags (fea_get_status) ---------------------------------- */
 #define FEA_STATUS_BLOWUP 1u       /* some u_i or v_i > 1e4 (CPUSolver.cpp:41-48) */
